@@ -136,6 +136,8 @@ struct TraceLaunch {
     int refill_below;         // refill a warp's idle lanes when fewer lanes are busy
     int postpone_pct;         // postpone triangles when fewer % of busy lanes have some
     int stack_limit;          // traversal stack entries a ray may use (1..kTraversalStack)
+    int tree_depth;           // node levels of the tree (bounds the depth-first stack)
+    int teams;                // the last rays of a warp are traced by teams of lanes (accel.cu)
     // Mixed launches only: an any-hit ray set traced in the same launch as
     // the closest-hit set above (same stride); its rays take indices
     // [0, *d_any_count) of the shared work counter.

@@ -223,6 +223,46 @@ __device__ __forceinline__ void visit(const float4 *__restrict__ nodes, uint32_t
     else visit_node<FMT == 2>(nodes, child, r, inv, oct, tmax, ng, tg);
 }
 
+// One child of a compressed node, tested by one lane of a team of eight: the
+// box test of visit_node for the child in `slot` (same planes, same slack),
+// with the node's other words that the team needs.  A node is 80 bytes, so
+// the team's loads of it fall into the same two or three sectors.
+__device__ __forceinline__ bool team_child(const float4 *__restrict__ nodes, uint32_t child, int slot,
+                                           const RayPre &r, V3 inv, int oct, float tmax, uint32_t &meta,
+                                           uint32_t &child_base, uint32_t &tri_base, uint32_t &imask) {
+    const float4 *np = nodes + 5 * (size_t)child;
+    const uint8_t *by = reinterpret_cast<const uint8_t *>(np) + slot;
+    const float4 q0 = __ldg(np);
+    const uint2 q1 = __ldg(reinterpret_cast<const uint2 *>(np + 1));
+    // planes of child `slot`: lo x, y, z at bytes 32, 40, 48, hi at 56, 64, 72
+    const int ox = (oct & 1) ? 56 : 32, oy = (oct & 2) ? 64 : 40, oz = (oct & 4) ? 72 : 48;
+    meta = __ldg(by + 24);
+    const uint32_t nx = __ldg(by + ox), fx = __ldg(by + 88 - ox);
+    const uint32_t ny = __ldg(by + oy), fy = __ldg(by + 104 - oy);
+    const uint32_t nz = __ldg(by + oz), fz = __ldg(by + 120 - oz);
+    const uint32_t ew = __float_as_uint(q0.w);
+    const float adx = __uint_as_float((ew & 0xffu) << 23) * inv.x;
+    const float ady = __uint_as_float(((ew >> 8) & 0xffu) << 23) * inv.y;
+    const float adz = __uint_as_float(((ew >> 16) & 0xffu) << 23) * inv.z;
+    const float cx = fmaf(-32768.f, adx, (q0.x - r.o.x) * inv.x);
+    const float cy = fmaf(-32768.f, ady, (q0.y - r.o.y) * inv.y);
+    const float cz = fmaf(-32768.f, adz, (q0.z - r.o.z) * inv.z);
+    const float dx = adx * 0.00390625f, dy = ady * 0.00390625f, dz = adz * 0.00390625f;
+    const float sx = fabsf(adx) * 0.015625f, sy = fabsf(ady) * 0.015625f, sz = fabsf(adz) * 0.015625f;
+    auto plane = [](uint32_t q) { return __uint_as_float(0x4B000000u | (q << 8)); };
+    const float tlimit = tmax + fabsf(tmax) * 5e-7f;
+    const int t0 = __vimax3_s32(__float_as_int(fmaf(plane(nx), dx, cx - sx)),
+                                __float_as_int(fmaf(plane(ny), dy, cy - sy)),
+                                max(__float_as_int(fmaf(plane(nz), dz, cz - sz)), __float_as_int(r.tmin)));
+    const int t1 = __vimin3_s32(__float_as_int(fmaf(plane(fx), dx, cx + sx)),
+                                __float_as_int(fmaf(plane(fy), dy, cy + sy)),
+                                min(__float_as_int(fmaf(plane(fz), dz, cz + sz)), __float_as_int(tlimit)));
+    child_base = q1.x;
+    tri_base = q1.y;
+    imask = ew >> 24;
+    return t0 <= t1 && meta != 0u;
+}
+
 __device__ __forceinline__ V3 box_inverse(V3 d) {
     float dx = fabsf(d.x) < 1e-20f ? copysignf(1e-20f, d.x) : d.x;
     float dy = fabsf(d.y) < 1e-20f ? copysignf(1e-20f, d.y) : d.y;
