@@ -10,6 +10,7 @@
 namespace krr {
 
 constexpr int kNrcMaxLevels = 16;
+constexpr int kNrcMaxLayers = 8;  // hidden layers (at most 7) and the output layer
 constexpr int kNrcIn = 64;       // padded MLP input width
 constexpr int kNrcWidth = 64;    // hidden width
 constexpr int kNrcOutPad = 16;   // padded output rows (3 used)
@@ -98,7 +99,7 @@ int nrc_backward_tc(const NrcMlp &mlp, const float *d_dy_out, const __nv_bfloat1
                     const int32_t *d_count, int64_t cap, const uint8_t *packed_wt, float *d_dx0,
                     float *d_dw, uint32_t *err, cudaStream_t s);
 int nrc_forward_tc(const NrcGrid &g, const NrcMlp &mlp, const float *d_in, const int32_t *d_count,
-                   int64_t cap, const __nv_bfloat16 *table, const uint8_t *packed, float *d_out,
+                   int64_t cap, const __nv_bfloat16 *table, const uint8_t *packed, float *d_out, int out_stride,
                    __nv_bfloat16 *acts, uint32_t *err, cudaStream_t s);
 int32_t nrc_train_stride(const krr_nrc *n);
 // Device word that is non-zero once a training step's loss was not finite:

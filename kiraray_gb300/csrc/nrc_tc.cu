@@ -1,17 +1,17 @@
 // Fused neural-radiance-cache forward pass on the 5th-generation tensor
-// cores (tcgen05), two 128-row tiles of queries in flight per CTA.
+// cores (tcgen05), one CTA per SM.
 //
-// Per tile: four encoder warps encode the queries (hash grid, trilinear)
-// into a 128x64 BF16 activation tile in shared memory while four MLP warps
-// run the previous tile: for each of the six layers one elected thread
-// issues four tcgen05.mma.kind::f16 (M=128, N=64 or 16, K=16, BF16 x BF16 ->
-// FP32 in tensor memory), commits them to an mbarrier, and the 128 MLP
-// threads read the accumulator rows back with tcgen05.ld, apply ReLU, round
-// to BF16 and write the next activation tile (or the RGB output).  All
-// weights (43 KB, BF16) stay resident in shared memory for the CTA's
-// lifetime.  Waits on the mbarrier are bounded: a wait that gives up sets an
-// error flag, and the CTA finishes without further tensor-core work and
-// frees its tensor memory.
+// Encoder warps encode the queries (hash grid, trilinear) into 128x64 BF16
+// activation tiles in shared memory while two groups of four MLP warps run
+// the tiles before them: for each layer one elected thread issues four
+// tcgen05.mma.kind::f16 (M=128, N=64 or 16, K=16, BF16 x BF16 -> FP32 in
+// tensor memory), commits them to an mbarrier, and the group's 128 threads
+// read the accumulator rows back with tcgen05.ld, apply ReLU, round to BF16
+// and write the next activation tile (or the RGB output).  All weights
+// (43 KB, BF16) stay resident in shared memory for the CTA's lifetime.
+// Waits on mbarriers are bounded: a wait that gives up sets an error flag,
+// and the CTA finishes without further tensor-core work and frees its tensor
+// memory.
 //
 // Shared-memory operands use the canonical K-major layout without swizzle:
 // 8x8-element core matrices of 128 contiguous bytes, core (i, j) of a tile
@@ -26,7 +26,6 @@ namespace krr {
 
 constexpr int kTcRows = 128;
 constexpr int kTcThreads = 128;
-constexpr uint32_t kTcCols = 64;                 // tensor-memory columns per CTA
 constexpr int kLayerBytes = kNrcWidth * kNrcIn * 2;     // 8 KB
 constexpr int kOutBytes = kNrcOutPad * kNrcIn * 2;      // 2 KB
 constexpr uint32_t kWaitLimit = 1u << 26;
@@ -141,118 +140,234 @@ __global__ void k_pack_weights(const __nv_bfloat16 *__restrict__ w, NrcMlp mlp, 
     }
 }
 
-// Hash-grid encoding of one query row.  The table gathers are the latency
-// of the whole kernel, so the levels go in groups of four: the 32 corner
-// loads of a group are issued before any of them is used (levels at or
-// beyond g.levels load entry 0 and are discarded), which turns sixteen
-// dependent round trips into four.  Per level the corner weights and the
-// accumulation order are those of the CUDA-core encoder (nrc.cu).
+// Hash-grid encoding of 16 query rows by one warp, two lanes per row: lane p
+// of a pair gathers the four corners at x offset p of four levels, then the
+// lanes swap halves, so that each interpolates two levels from all eight
+// corners and stores their four features.  The two x neighbours of a corner
+// pair lie next to each other in the table (a hashed index is x ^ (a function
+// of y and z), a dense one x + (the same)), in one 32-byte sector seven times
+// in eight, so a pair's two loads, issued by one instruction, share an L1
+// request.  Per level the corner weights and the accumulation order are those
+// of the CUDA-core encoder (nrc.cu).
 constexpr int kEncGroup = 4;
 
-__device__ __forceinline__ void encode_row(const NrcGrid &g, const float *q,
-                                           const __nv_bfloat16 *__restrict__ table, float *x) {
-    float p[3];
-    for (int a = 0; a < 3; ++a) p[a] = fminf(fmaxf((q[a] - g.lo[a]) * g.inv_extent[a], 0.f), 1.f);
-#pragma unroll 1
-    for (int l0 = 0; l0 < kNrcMaxLevels; l0 += kEncGroup) {
-        if (l0 >= g.levels) break;
-        __nv_bfloat162 v[kEncGroup][8];
-        float fr[kEncGroup][3];
+struct EncInput {
+    float pos[3], dir[3], mat[3];   // dir: normal (lane 0) or outgoing direction (lane 1); mat: roughness or albedo
+};
+
+__device__ __forceinline__ EncInput load_input(const float *q, int p) {
+    EncInput x;
 #pragma unroll
-        for (int j = 0; j < kEncGroup; ++j) {
-            const int l = l0 + j;
-            const bool valid = l < g.levels;
-            uint32_t base[3];
-            for (int a = 0; a < 3; ++a) {
-                float s = p[a] * (float)g.res[l];
-                float fl = fminf(fmaxf(floorf(s), 0.f), (float)(g.res[l] - 1));
-                base[a] = (uint32_t)fl;
-                fr[j][a] = fminf(fmaxf(s - fl, 0.f), 1.f);
-            }
-            uint32_t n1 = (uint32_t)g.res[l] + 1u;
-            bool dense = g.dense_mask & (1u << l);
+    for (int a = 0; a < 3; ++a) {
+        x.pos[a] = q[a];
+        x.dir[a] = q[(p ? 10 : 3) + a];
+    }
+    x.mat[0] = q[p ? 7 : 6];
+    x.mat[1] = p ? q[8] : 0.f;
+    x.mat[2] = p ? q[9] : 0.f;
+    return x;
+}
+
+__device__ __forceinline__ uint32_t bf16x2(float a, float b) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t *>(&v);
+}
+
+// The lane's four corners (y, z) = 00, 10, 01, 11 of levels l0..l0+3; a level
+// at or beyond g.levels reads entry 0 and is discarded.
+__device__ __forceinline__ void gather_levels(const NrcGrid &g, const float *pos, const __nv_bfloat16 *__restrict__ table,
+                                              int l0, uint32_t p, uint32_t (&v)[kEncGroup][4]) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                uint32_t xx = base[0] + (k & 1), yy = base[1] + ((k >> 1) & 1), zz = base[2] + ((k >> 2) & 1);
-                uint32_t idx = dense ? xx + n1 * (yy + n1 * zz)
-                                     : (xx ^ (yy * 2654435761u) ^ (zz * 805459861u)) & (g.table_size - 1u);
-                idx = valid ? idx + g.offset[l] : 0u;
-                v[j][k] = *reinterpret_cast<const __nv_bfloat162 *>(table + 2 * (size_t)idx);
-            }
+    for (int j = 0; j < kEncGroup; ++j) {
+        const int l = (l0 + j) & (kNrcMaxLevels - 1);
+        const bool valid = l0 + j < g.levels;
+        const char *level = reinterpret_cast<const char *>(table) + 4 * (size_t)(valid ? g.offset[l] : 0u);
+        const float res = (float)g.res[l], top = (float)(g.res[l] - 1);
+        uint32_t c[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) c[a] = (uint32_t)fminf(fmaxf(floorf(pos[a] * res), 0.f), top);
+        // byte offsets: the factor 4 goes into the multipliers and the mask
+        const uint32_t x = 4u * (c[0] + p);
+        uint32_t off[4];
+        if (g.dense_mask & (1u << l)) {
+            const uint32_t n1 = 4u * ((uint32_t)g.res[l] + 1u), n2 = n1 * ((uint32_t)g.res[l] + 1u);
+            off[0] = x + c[1] * n1 + c[2] * n2;
+            off[1] = off[0] + n1;
+            off[2] = off[0] + n2;
+            off[3] = off[1] + n2;
+        } else {
+            const uint32_t mask = valid ? 4u * (g.table_size - 1u) : 0u;
+            const uint32_t y0 = c[1] * (4u * 2654435761u), z0 = c[2] * (4u * 805459861u);
+            const uint32_t y1 = y0 + 4u * 2654435761u, z1 = z0 + 4u * 805459861u;
+            off[0] = (x ^ y0 ^ z0) & mask;
+            off[1] = (x ^ y1 ^ z0) & mask;
+            off[2] = (x ^ y0 ^ z1) & mask;
+            off[3] = (x ^ y1 ^ z1) & mask;
         }
 #pragma unroll
-        for (int j = 0; j < kEncGroup; ++j) {
-            if (l0 + j >= g.levels) break;
+        for (int k = 0; k < 4; ++k) v[j][k] = __ldg(reinterpret_cast<const uint32_t *>(level + off[k]));
+    }
+}
+
+// Row r of the tile; p: the lane's place in the row's pair.  Warp-collective.
+__device__ __forceinline__ void encode_row(const NrcGrid &g, const EncInput &in,
+                                           const __nv_bfloat16 *__restrict__ table, uint8_t *tile, uint32_t r,
+                                           uint32_t p) {
+    float pos[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) pos[a] = fminf(fmaxf((in.pos[a] - g.lo[a]) * g.inv_extent[a], 0.f), 1.f);
+#pragma unroll 1
+    for (int l0 = 0; l0 < g.levels; l0 += kEncGroup) {
+        uint32_t v[kEncGroup][4];
+        gather_levels(g, pos, table, l0, p, v);
+        // lane 0 keeps levels l0, l0+1 and takes their x + 1 corners, lane 1
+        // keeps l0+2, l0+3 and takes their x corners
+        const int first = l0 + 2 * (int)p;
+        uint32_t f[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            uint32_t c[8];   // corner k at bits x | y << 1 | z << 2
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t mine = p ? v[j + 2][k] : v[j][k], other = p ? v[j][k] : v[j + 2][k];
+                const uint32_t got = __shfl_xor_sync(0xffffffffu, other, 1);
+                c[2 * k] = p ? got : mine;
+                c[2 * k + 1] = p ? mine : got;
+            }
+            const int l = (l0 + j) & (kNrcMaxLevels - 1), l2 = (l0 + j + 2) & (kNrcMaxLevels - 1);
+            const float res = (float)(p ? g.res[l2] : g.res[l]), top = (float)((p ? g.res[l2] : g.res[l]) - 1);
+            float fr[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float s = pos[a] * res;
+                fr[a] = __saturatef(s - fminf(fmaxf(floorf(s), 0.f), top));
+            }
             float f0 = 0.f, f1 = 0.f;
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                float w = ((k & 1) ? fr[j][0] : 1.f - fr[j][0]) *
-                          (((k >> 1) & 1) ? fr[j][1] : 1.f - fr[j][1]) *
-                          (((k >> 2) & 1) ? fr[j][2] : 1.f - fr[j][2]);
-                f0 += w * __bfloat162float(v[j][k].x);
-                f1 += w * __bfloat162float(v[j][k].y);
+                const float w = ((k & 1) ? fr[0] : 1.f - fr[0]) * (((k >> 1) & 1) ? fr[1] : 1.f - fr[1]) *
+                                (((k >> 2) & 1) ? fr[2] : 1.f - fr[2]);
+                f0 += w * __uint_as_float(c[k] << 16);
+                f1 += w * __uint_as_float(c[k] & 0xffff0000u);
             }
-            x[2 * (l0 + j)] = f0;
-            x[2 * (l0 + j) + 1] = f1;
+            f[j] = bf16x2(f0, f1);
         }
+        uint8_t *dst = tile + canon(r, 2u * (uint32_t)first);
+        if (first + 2 <= g.levels) *reinterpret_cast<uint2 *>(dst) = make_uint2(f[0], f[1]);
+        else if (first < g.levels) *reinterpret_cast<uint32_t *>(dst) = f[0];
     }
-    int o = 2 * g.levels;
-    nrc_encode_extras(q, x + o);
-    for (int k = o + kNrcExtra; k < kNrcIn; ++k) x[k] = 0.f;
+    // the other inputs, as nrc_encode_extras: lane 0 the normal and the
+    // roughness, lane 1 the outgoing direction and the albedo; zeros behind
+    const uint32_t o = 2u * (uint32_t)g.levels;
+    auto put = [&](uint32_t k, float a, float b) {
+        *reinterpret_cast<uint32_t *>(tile + canon(r, k)) = bf16x2(a, b);
+    };
+    float t, u, e[kNrcBlobBins];
+    nrc_spherical(in.dir[0], in.dir[1], in.dir[2], t, u);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        nrc_one_blob(k ? u : t, e);
+        put(o + 8u * p + 4u * k, e[0], e[1]);
+        put(o + 8u * p + 4u * k + 2u, e[2], e[3]);
+    }
+    if (p == 0) {
+        nrc_one_blob(1.f - expf(-in.mat[0]), e);
+        put(o + 16u, e[0], e[1]);
+        put(o + 18u, e[2], e[3]);
+    } else {
+        put(o + 20u, in.mat[0], in.mat[1]);
+        put(o + 22u, in.mat[2], 0.f);
+    }
+    for (uint32_t k = o + 24u + 2u * p; k < (uint32_t)kNrcIn; k += 4u) put(k, 0.f, 0.f);
 }
 
-__device__ __forceinline__ void bar_sync(int id, int n) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
-}
-__device__ __forceinline__ void bar_arrive(int id, int n) {
-    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+// Named barrier of n threads; true for all of them if `flag` is for one.
+__device__ __forceinline__ bool bar_or(int id, int n, bool flag) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %3, 0;\n\tbar.red.or.pred p, %1, %2, q;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(r)
+        : "r"(id), "r"(n), "r"((uint32_t)flag)
+        : "memory");
+    return r != 0u;
 }
 
-// Named barriers of the forward kernel (0 is __syncthreads): a tile buffer
-// is full (encoders -> MLP warps), a tile buffer is free again (MLP warps
-// -> encoders), and the MLP warps' own per-layer barrier.
-constexpr int kBarFull = 1, kBarEmpty = 3, kBarMlp = 5;
-constexpr int kFwThreads = 256;   // warps 0-3: MLP (tensor-memory lanes 0-127); 4-7: encoders
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+}
 
-// out[i][0..3) for i < *count (or cap); optional per-layer activation dump
-// (bf16 [layers][cap][64], row-major) for the training backward pass.
+// Bounded wait of a whole warp, one outcome for its lanes.
+__device__ __forceinline__ bool warp_wait(uint32_t mbar, uint32_t parity) {
+    uint32_t spins = 0, ok = 0;
+    while (!(ok = mbar_try_wait(mbar, parity)) && ++spins < kWaitLimit) {
+    }
+    return __all_sync(0xffffffffu, ok);
+}
+
+// One CTA of 32 warps per SM: 8 MLP warps in two groups (tensor-memory lanes
+// 0-127 each, 64 columns apart) and 24 encoder warps, with kTileBuffers
+// activation tiles between them.  64 registers a thread; the weights and the
+// tiles take 122 KB of shared memory (five hidden layers), which leaves half
+// of the SM's L1 to the table.
+constexpr int kMlpGroups = 2, kEncWarps = 24, kTileBuffers = 5;
+constexpr int kTileBytes = kTcRows * kNrcIn * 2;
+constexpr int kUnitsPerTile = kTcRows / 16;   // an encoder warp's unit of work: 16 rows
+constexpr int kFwThreads = kMlpGroups * kTcRows + 32 * kEncWarps;
+constexpr uint32_t kFwCols = 64u * kMlpGroups;
+
+// out[i * out_stride + 0..3) for i < *count (or cap); optional per-layer
+// activation dump (bf16 [layers][cap][64], row-major) for the training
+// backward pass.
 //
-// Warp-specialised: warps 4-7 encode the rows of the CTA's next tile (the
-// hash-grid gathers) into one of two activation buffers while warps 0-3 run
-// the six layers of the current tile out of the other (one thread issues
-// the MMAs, all 128 read the accumulator rows back, apply ReLU and write the
-// next layer's input in place), so the gathers of tile k+1 overlap the MMA
-// chain of tile k.  The groups hand the buffers over with named barriers;
-// after a failed (bounded) accumulator wait the MLP warps skip the compute
-// of the remaining tiles but keep handing buffers back, so no warp waits
-// forever.
+// Warp-specialised: the encoder warps fill tiles of 128 rows (the hash-grid
+// gathers), 16 rows at a time, while each MLP group runs the layers of every
+// second tile (one thread issues the MMAs, all 128 read the accumulator rows
+// back, apply ReLU and write the next layer's input in place).  Tiles are
+// handed over by mbarriers: full (eight 16-row units encoded) and empty (the
+// group's four warps are done).
+//
+// An SM takes one L1 miss per clock (296 G/s over the chip with the table in
+// L2, whatever the loads' kind and the warps in flight), and a query misses
+// about 50 times: 0.26 ms for 1.5M queries.  Those take 397 us; 824 us with
+// one lane per row, four encoder warps and a CTA-wide handover (two CTAs of
+// 8 warps), 618 us with two lanes per row and two CTAs of 8 encoder warps:
+// then the loads' latency was the limit, and 24 encoder warps on 64 registers
+// hide it better than deeper batches of loads in 16.
+// Waits are bounded: a group (or an encoder warp) whose wait gives up raises
+// an error flag and leaves, as do in turn those that wait for it.
 __global__ void __launch_bounds__(kFwThreads, 1)
 k_nrc_forward_tc(NrcGrid g, int layers, const float *__restrict__ in, const int32_t *d_count,
                  int64_t cap, const __nv_bfloat16 *__restrict__ table,
-                 const uint8_t *__restrict__ packed_w, float *__restrict__ out,
+                 const uint8_t *__restrict__ packed_w, float *__restrict__ out, int out_stride,
                  __nv_bfloat16 *__restrict__ acts, uint32_t *err) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *sw = smem;                                              // weights
-    uint8_t *sa0 = smem + (layers - 1) * kLayerBytes + kOutBytes;    // activation tiles
-    sa0 = reinterpret_cast<uint8_t *>(((uintptr_t)sa0 + 1023) & ~(uintptr_t)1023);
-    uint8_t *sa1 = sa0 + kTcRows * kNrcIn * 2;
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(sa1 + kTcRows * kNrcIn * 2);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mbar + 1);
-    uint32_t *fail_flag = tmem_slot + 1;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    uint8_t *tiles_s = smem + (layers - 1) * kLayerBytes + kOutBytes;   // activation tiles
+    tiles_s = reinterpret_cast<uint8_t *>(((uintptr_t)tiles_s + 1023) & ~(uintptr_t)1023);
+    uint64_t *mbars = reinterpret_cast<uint64_t *>(tiles_s + kTileBuffers * kTileBytes);
+    const uint32_t full0 = smem_u32(mbars), empty0 = full0 + 8 * kTileBuffers,
+                   acc0 = empty0 + 8 * kTileBuffers;   // acc: a group's accumulator is complete
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mbars + 2 * kTileBuffers + kMlpGroups);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
     // weights -> shared memory (16-byte copies)
     int wbytes = (layers - 1) * kLayerBytes + kOutBytes;
     for (int e = tid; e < wbytes / 16; e += blockDim.x)
         reinterpret_cast<uint4 *>(sw)[e] = reinterpret_cast<const uint4 *>(packed_w)[e];
+    fence_proxy_async();   // the tensor cores read the weights through the async proxy
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(tmem_slot)),
-                     "r"(kTcCols));
+                     "r"(kFwCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        mbar_init(smem_u32(mbar), 1);
+        for (int b = 0; b < kTileBuffers; ++b) {
+            mbar_init(full0 + 8 * b, kUnitsPerTile);
+            mbar_init(empty0 + 8 * b, kTcRows / 32);
+        }
+        for (int m = 0; m < kMlpGroups; ++m) mbar_init(acc0 + 8 * m, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     fence_before_sync();
@@ -262,103 +377,109 @@ k_nrc_forward_tc(NrcGrid g, int layers, const float *__restrict__ in, const int3
 
     const int64_t n = d_count ? min((int64_t)*d_count, cap) : cap;
     const int64_t tiles = (n + kTcRows - 1) / kTcRows;
-    if (warp >= 4) {
-        // encoders: row r of each tile into the free buffer
-        const int r = tid - 128;
-        float x[kNrcIn];
-        int k = 0;
-        for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x, ++k) {
-            uint8_t *sa = (k & 1) ? sa1 : sa0;
-            if (k >= 2) bar_sync(kBarEmpty + (k & 1), kFwThreads);
-            const int64_t row = t * kTcRows + r;
-            if (row < n) encode_row(g, in + kNrcInputs * row, table, x);
-            else
-                for (int q = 0; q < kNrcIn; ++q) x[q] = 0.f;
-            store_row(sa, (uint32_t)r, x);
+    // the CTA's k-th tile is tile blockIdx.x + k gridDim.x, in buffer
+    // k % kTileBuffers; a buffer's k / kTileBuffers-th use flips the parity
+    if (warp >= 4 * kMlpGroups) {
+        // encoders: a warp's rows are 16 of each third tile (rows past the
+        // last are encoded as the last: their results are never stored)
+        const int e = warp - 4 * kMlpGroups;
+        const uint32_t r = (uint32_t)((e % kUnitsPerTile) * 16 + (lane >> 1)), p = (uint32_t)lane & 1u;
+        for (int k = e / kUnitsPerTile;; k += kEncWarps / kUnitsPerTile) {
+            const int64_t t = blockIdx.x + (int64_t)k * gridDim.x;
+            if (t >= tiles) break;
+            const int64_t row = min(t * kTcRows + r, n - 1);
+            const EncInput x = load_input(in + kNrcInputs * row, (int)p);
+            const int b = k % kTileBuffers;
+            if (!warp_wait(empty0 + 8 * b, (uint32_t)(k / kTileBuffers + 1) & 1u)) {
+                if (lane == 0) atomicOr(err, (uint32_t)kErrLoopLimit);
+                break;
+            }
+            encode_row(g, x, table, tiles_s + b * kTileBytes, r, p);
             fence_proxy_async();   // the tensor cores read the tile through the async proxy
-            bar_arrive(kBarFull + (k & 1), kFwThreads);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full0 + 8 * b);
         }
     } else {
-        const uint32_t my_lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
+        const int m = warp >> 2, row_t = tid & (kTcRows - 1);
+        const uint32_t acc = acc0 + 8 * m, d_cols = tmem + 64u * m;
+        const uint32_t my_lane_addr = d_cols + ((uint32_t)((warp & 3) * 32) << 16);
         uint32_t phase = 0;
         bool failed = false;
-        int k = 0;
-        for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x, ++k) {
-            uint8_t *sa = (k & 1) ? sa1 : sa0;
-            bar_sync(kBarFull + (k & 1), kFwThreads);
-            const int64_t row = t * kTcRows + tid;
-            for (int l = 0; l < layers && !failed; ++l) {
+        for (int k = m; !failed; k += kMlpGroups) {
+            const int64_t t = blockIdx.x + (int64_t)k * gridDim.x;
+            if (t >= tiles) break;
+            const int b = k % kTileBuffers;
+            uint8_t *sa = tiles_s + b * kTileBytes;
+            failed = !warp_wait(full0 + 8 * b, (uint32_t)(k / kTileBuffers) & 1u);
+            const int64_t row = t * kTcRows + row_t;
+            for (int l = 0; l < layers; ++l) {
                 const bool last = l + 1 == layers;
-                const int nrows = last ? kNrcOutPad : kNrcWidth;
-                // the tile holds this layer's input X_l: dump it for the
-                // backward pass while the MMAs read it (it is overwritten
-                // only after the accumulator wait's barrier)
+                if (row_t == 0 && !failed) {
+                    fence_after_sync();
+                    const uint32_t a0 = smem_u32(sa), b0 = smem_u32(sw + l * kLayerBytes);
+                    const uint32_t idesc = idesc_bf16(kTcRows, last ? kNrcOutPad : kNrcWidth);
+#pragma unroll
+                    for (int kk = 0; kk < kNrcIn / 16; ++kk)
+                        tc_mma(d_cols, smem_desc(a0 + 256u * kk, 128u, 1024u),
+                               smem_desc(b0 + 256u * kk, 128u, 1024u), idesc, kk > 0 ? 1u : 0u);
+                    tc_commit(acc);
+                }
+                __syncwarp();
+                // the tile holds this layer's input X_l: the warp dumps its
+                // own 32 rows for the backward pass while the MMAs read them
+                // (it alone overwrites these rows, below)
                 if (acts) {
                     __nv_bfloat16 *dst = acts + (size_t)l * cap * kNrcIn;
-                    for (int c = tid; c < kTcRows * 8; c += kTcRows) {
-                        const int rr = c >> 3, j = c & 7;
+                    for (int c = lane; c < 32 * 8; c += 32) {
+                        const int rr = (warp & 3) * 32 + (c >> 3), j = c & 7;
                         if (t * kTcRows + rr < n)
                             reinterpret_cast<uint4 *>(dst + (t * kTcRows + rr) * kNrcIn)[j] =
                                 *reinterpret_cast<const uint4 *>(sa + canon((uint32_t)rr, (uint32_t)(8 * j)));
                     }
+                    __syncwarp();
                 }
-                if (tid == 0) {
-                    fence_after_sync();
-                    const uint32_t a0 = smem_u32(sa), b0 = smem_u32(sw + l * kLayerBytes);
-                    const uint32_t idesc = idesc_bf16(kTcRows, nrows);
-#pragma unroll
-                    for (int kk = 0; kk < kNrcIn / 16; ++kk)
-                        tc_mma(tmem, smem_desc(a0 + 256u * kk, 128u, 1024u),
-                               smem_desc(b0 + 256u * kk, 128u, 1024u), idesc, kk > 0 ? 1u : 0u);
-                    tc_commit(smem_u32(mbar));
-                    // bounded wait for the accumulator; the decision to stop
-                    // is uniform across the MLP warps
-                    uint32_t spins = 0, ok = 0;
-                    while (!(ok = mbar_try_wait(smem_u32(mbar), phase)) && ++spins < kWaitLimit) {
-                    }
-                    *fail_flag = ok ? 0u : 1u;
-                    if (!ok) atomicOr(err, (uint32_t)kErrLoopLimit);
-                }
-                bar_sync(kBarMlp, kTcRows);
-                if (*fail_flag) {
-                    failed = true;
-                    break;
-                }
-                {
-                    uint32_t spins = 0;   // already complete: returns at once
-                    while (!mbar_try_wait(smem_u32(mbar), phase) && ++spins < kWaitLimit) {
-                    }
-                }
+                if (!failed) failed = !warp_wait(acc, phase);
                 phase ^= 1u;
-                fence_after_sync();
-                float v[kNrcIn];
-                tmem_ld16(my_lane_addr + 0, v);
-                if (!last) {
-                    tmem_ld16(my_lane_addr + 16, v + 16);
-                    tmem_ld16(my_lane_addr + 32, v + 32);
-                    tmem_ld16(my_lane_addr + 48, v + 48);
-                }
-                tmem_wait_ld();
-                if (!last) {
-                    for (int q = 0; q < kNrcIn; ++q) v[q] = fmaxf(v[q], 0.f);
-                    store_row(sa, (uint32_t)tid, v);
-                    fence_proxy_async();
-                } else if (row < n) {
-                    out[row * kNrcOutPad + 0] = v[0];
-                    out[row * kNrcOutPad + 1] = v[1];
-                    out[row * kNrcOutPad + 2] = v[2];
+                if (!failed) {
+                    fence_after_sync();
+                    if (!last) {
+#pragma unroll
+                        for (int h = 0; h < 4; ++h) {   // 16 columns at a time
+                            float v[16];
+                            tmem_ld16(my_lane_addr + 16 * h, v);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int q = 0; q < 16; ++q) v[q] = fmaxf(v[q], 0.f);
+#pragma unroll
+                            for (int j = 0; j < 2; ++j)
+                                *reinterpret_cast<uint4 *>(sa + canon((uint32_t)row_t, 16u * h + 8u * j)) =
+                                    make_uint4(bf16x2(v[8 * j], v[8 * j + 1]), bf16x2(v[8 * j + 2], v[8 * j + 3]),
+                                               bf16x2(v[8 * j + 4], v[8 * j + 5]), bf16x2(v[8 * j + 6], v[8 * j + 7]));
+                        }
+                        fence_proxy_async();
+                    } else {
+                        float v[16];
+                        tmem_ld16(my_lane_addr, v);
+                        tmem_wait_ld();
+                        if (row < n) {
+                            out[row * out_stride + 0] = v[0];
+                            out[row * out_stride + 1] = v[1];
+                            out[row * out_stride + 2] = v[2];
+                        }
+                    }
                 }
                 fence_before_sync();
-                bar_sync(kBarMlp, kTcRows);
+                failed = bar_or(1 + m, kTcRows, failed);   // one outcome for the group
             }
-            bar_arrive(kBarEmpty + (k & 1), kFwThreads);   // the buffer is free
+            if (lane == 0) mbar_arrive(empty0 + 8 * b);
         }
+        if (failed && lane == 0) atomicOr(err, (uint32_t)kErrLoopLimit);
     }
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcCols));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kFwCols));
 }
 
 // ------------------------------------------------------------------ backward
@@ -579,32 +700,10 @@ k_nrc_backward_tc(int layers, const float *__restrict__ dy_out, const __nv_bfloa
 
 }  // namespace
 
-// Resident CTAs per SM of a tensor-memory kernel, from its registers, its
-// shared memory (carveout at the maximum) and its tensor-memory columns.
-// (The occupancy query does not count tensor memory and reported one CTA
-// for this kernel, the carveout preference not yet applied.)
-static int tc_ctas_per_sm(const void *fn, int threads, size_t smem, int dev) {
-    cudaFuncAttributes fa{};
-    int regs_sm = 0, smem_sm = 0, smem_reserved = 0, threads_sm = 0;
-    if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess ||
-        cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&smem_reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&threads_sm, cudaDevAttrMaxThreadsPerMultiProcessor, dev) != cudaSuccess) {
-        cudaGetLastError();
-        return 1;
-    }
-    const int by_regs = regs_sm / std::max(1, threads * std::max(1, fa.numRegs));
-    const int by_smem = smem_sm / (int)std::max<size_t>(1, smem + fa.sharedSizeBytes + smem_reserved);
-    const int by_threads = threads_sm / threads;
-    const int by_tmem = 512 / (int)kTcCols;
-    return std::max(1, std::min(std::min(by_regs, by_smem), std::min(by_threads, by_tmem)));
-}
-
 size_t nrc_tc_smem_bytes(int layers) {
     size_t w = (size_t)(layers - 1) * kLayerBytes + kOutBytes;
-    size_t a = ((w + 1023) & ~(size_t)1023) + 2 * kTcRows * kNrcIn * 2;   // two tile buffers
-    return a + 64 + 1024;   // mbarrier, tensor-memory slot, alignment slack
+    size_t a = ((w + 1023) & ~(size_t)1023) + kTileBuffers * kTileBytes;
+    return a + 128 + 1024;   // mbarriers, tensor-memory slot, alignment slack
 }
 
 int nrc_pack_weights(const __nv_bfloat16 *w, const NrcMlp &mlp, uint8_t *packed, cudaStream_t s) {
@@ -633,7 +732,7 @@ int nrc_backward_tc(const NrcMlp &mlp, const float *d_dy_out, const __nv_bfloat1
     size_t smem = nrc_tc_bwd_smem_bytes(mlp.layers);
     if (!configured) {
         KRR_CUDA(cudaFuncSetAttribute(k_nrc_backward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+                                      (int)nrc_tc_bwd_smem_bytes(kNrcMaxLayers)));
         configured = true;
     }
     int dev = 0, sms = 0;
@@ -648,30 +747,22 @@ int nrc_backward_tc(const NrcMlp &mlp, const float *d_dy_out, const __nv_bfloat1
 }
 
 int nrc_forward_tc(const NrcGrid &g, const NrcMlp &mlp, const float *d_in, const int32_t *d_count,
-                   int64_t cap, const __nv_bfloat16 *table, const uint8_t *packed, float *d_out,
+                   int64_t cap, const __nv_bfloat16 *table, const uint8_t *packed, float *d_out, int out_stride,
                    __nv_bfloat16 *acts, uint32_t *err, cudaStream_t s) {
     static bool configured = false;
     size_t smem = nrc_tc_smem_bytes(mlp.layers);
-    if (!configured) {
+    if (!configured) {   // for the deepest network, whatever this one's depth
         KRR_CUDA(cudaFuncSetAttribute(k_nrc_forward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-        // the largest shared-memory carveout, so that several CTAs fit
-        KRR_CUDA(cudaFuncSetAttribute(k_nrc_forward_tc, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                      cudaSharedmemCarveoutMaxShared));
+                                      (int)nrc_tc_smem_bytes(kNrcMaxLayers)));
         configured = true;
     }
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // several CTAs per SM, so that the hash gathers of one CTA's tile overlap
-    // the MMA chains of the others: as many as registers, shared memory and
-    // the 512 tensor-memory columns allow (3 for five hidden layers)
-    static int per_sm = 0;
-    if (!per_sm) per_sm = tc_ctas_per_sm((const void *)k_nrc_forward_tc, kFwThreads, smem, dev);
     int64_t tiles = (cap + kTcRows - 1) / kTcRows;
-    int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)sms * per_sm));
+    int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)sms));
     k_nrc_forward_tc<<<grid, kFwThreads, smem, s>>>(g, mlp.layers, d_in, d_count, cap, table, packed,
-                                                    d_out, acts, err);
+                                                    d_out, out_stride, acts, err);
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }

@@ -1,0 +1,57 @@
+"""The cache's hash-grid gathers, two lanes to a row, at the edges of their
+groups: levels that do not fill a group of four, dense and hashed levels in
+one group, row counts around a tile and a warp's rows, and the activations
+that training keeps of such tiles."""
+import numpy as np
+import pytest
+import torch
+
+from kiraray_gb300.nrc import NeuralRadianceCache
+from oracle import nrc_ref as R
+from tests.test_nrc_gpu import _oracle, _records, _rel, _targets
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("levels,log2_table,hidden", [(1, 14, 1), (3, 10, 2), (4, 14, 5), (5, 8, 3), (8, 12, 2),
+                                                      (9, 12, 5), (13, 14, 6), (16, 10, 5)])
+def test_levels_and_rows(krr_lib, cuda, levels, log2_table, hidden):
+    """Predictions against the CUDA-core kernels.  Both encode in the same
+    order of operations, and round to BF16 (2^-9) at the same places; only the
+    FP32 sums of the layers differ, so that an activation may round the other
+    way: 2^-8 of the norm bounds that with room."""
+    kw = dict(n_levels=levels, log2_table_size=log2_table, base_resolution=4, max_resolution=300,
+              hidden_layers=hidden)
+    tc = NeuralRadianceCache((-1, -1, -1), (1, 1, 1), tensor_cores=1, **kw)
+    ref = NeuralRadianceCache((-1, -1, -1), (1, 1, 1), tensor_cores=0, **kw)
+    rng = np.random.default_rng(levels)
+    table = (rng.random(tc.params(1).size, dtype=np.float32) - np.float32(0.5))
+    for c in (tc, ref):
+        c.set_params(0, ref.params(0))
+        c.set_params(1, table)
+    q = torch.from_numpy(_records(1000, levels)).cuda()
+    whole = tc.query(q).cpu().numpy()
+    assert _rel(whole, ref.query(q).cpu().numpy()) < 2.0 ** -8
+    for n in (1, 15, 16, 17, 127, 128, 129, 999):
+        assert np.array_equal(tc.query(q[:n].contiguous()).cpu().numpy(), whole[:n]), n
+
+
+@pytest.mark.parametrize("n", [1, 17, 130, 3001])
+@pytest.mark.parametrize("levels", [1, 7, 16])
+def test_table_gradient(krr_lib, cuda, levels, n):
+    """The gradient that the kept activations give, against the oracle's (64
+    bits, BF16 rounding of the layers' operands): 3e-2 of the norm, as for the
+    trained cache."""
+    cache = NeuralRadianceCache((-1, -1, -1), (1, 1, 1), n_levels=levels, log2_table_size=10, base_resolution=4,
+                                max_resolution=200)
+    rng = np.random.default_rng(n)
+    cache.set_params(1, (rng.random(cache.params(1).size, dtype=np.float32) - np.float32(0.5)))
+    rec = _records(n, n)
+    tgt = _targets(rec)
+    _, gt, _ = cache.gradients(torch.from_numpy(rec).cuda(), torch.from_numpy(tgt).cuda())
+    grid, mlp, table, info = _oracle(cache, (-1, -1, -1), (1, 1, 1))
+    X0, cs = R.encode(grid, table, rec)
+    y, acts = R.forward(mlp, X0)
+    _, dy = R.loss_and_grad(y, tgt.astype(np.float64))
+    _, dX0 = R.backward(mlp, acts, dy, loss_scale=cache.cfg.loss_scale)
+    assert _rel(gt, R.table_grad(grid, cs, dX0, info.n_table_entries)) < 3e-2
