@@ -44,7 +44,6 @@ struct krr_nrc {
     float *loss = nullptr;                   // device loss accumulator
     int32_t *count_buf = nullptr;
     uint8_t *packed = nullptr;               // weights in tcgen05 canonical tiles
-    uint8_t *packed_t = nullptr;             // transposed weights (backward)
     uint32_t *err = nullptr;                 // device error flags
     // inference copy (ema_decay > 0): exponential moving average of the
     // parameters after each Adam step, FP32 and BF16, and its packed tiles;
@@ -525,15 +524,15 @@ int backward(krr_nrc *n, const float *d_inputs, const float *d_targets, const in
              int64_t cap, cudaStream_t s) {
     const float scale = n->cfg.loss_scale;
     KRR_CUDA(cudaMemsetAsync(n->loss, 0, sizeof(float), s));
-    k_loss<<<grid_for(cap), kThreads, 0, s>>>(n->out, d_targets, d_count, cap, scale, n->dA, n->loss);
-    KRR_CUDA(cudaGetLastError());
     float *dY = n->dA, *dX = n->dB;
-    if (n->cfg.tensor_cores) {
-        // dX0 -> dB, dW += on the tensor cores
-        KRR_TRY(nrc_backward_tc(n->mlp, n->dA, n->act, d_count, cap, n->packed_t, n->dB, n->w_grad,
-                                n->err, s));
+    if (n->cfg.tensor_cores && n->mlp.layers <= kNrcTcBwdLayers) {
+        // loss, dX0 -> dB, dW += on the tensor cores
+        KRR_TRY(nrc_backward_tc(n->mlp, 2 * n->grid.levels, n->out, d_targets, scale, n->act, d_count, cap,
+                                n->packed, n->dB, n->w_grad, n->loss, n->err, s));
         dY = n->dB;
     } else {
+        k_loss<<<grid_for(cap), kThreads, 0, s>>>(n->out, d_targets, d_count, cap, scale, n->dA, n->loss);
+        KRR_CUDA(cudaGetLastError());
         // backward through the layers: dY holds the gradient of layer l's output
         int blocks = grid_for(cap, 128);
         int wblocks = grid_for(cap, 64);
@@ -562,13 +561,13 @@ int backward(krr_nrc *n, const float *d_inputs, const float *d_targets, const in
     return KRR_OK;
 }
 
-// Both weight layouts of the tensor-core kernels, from the BF16 weights, and
-// the forward layout of the inference copy.
+// The tensor-core kernels' layout of the BF16 weights, and of the inference
+// copy's.
 int pack_weights(krr_nrc *n, cudaStream_t s) {
     if (!n->cfg.tensor_cores) return KRR_OK;
     KRR_TRY(nrc_pack_weights(n->weights, n->mlp, n->packed, s));
     if (n->ema_w) KRR_TRY(nrc_pack_weights(n->ema_weights, n->mlp, n->ema_packed, s));
-    return nrc_pack_weights_t(n->weights, n->mlp, n->packed_t, s);
+    return KRR_OK;
 }
 
 // The inference copy restarts from the trained parameters.
@@ -707,7 +706,6 @@ extern "C" int krr_nrc_create(const krr_nrc_config *cfg, krr_nrc **out) {
     alloc((void **)&n->table, tn * 2);
     alloc((void **)&n->loss, 16);
     alloc((void **)&n->packed, (size_t)(m.layers - 1) * kNrcWidth * kNrcIn * 2 + kNrcOutPad * kNrcIn * 2);
-    alloc((void **)&n->packed_t, (size_t)(m.layers - 1) * kNrcWidth * kNrcIn * 2 + kNrcIn * kNrcOutPad * 2);
     alloc((void **)&n->err, 16);
     alloc((void **)&n->step, 16);
     if (cfg->ema_decay > 0.f) {
@@ -742,7 +740,7 @@ extern "C" int krr_nrc_destroy(krr_nrc *n) {
                     (void *)n->table_grad, (void *)n->table, (void *)n->w_master, (void *)n->w_m,
                     (void *)n->w_v, (void *)n->w_grad, (void *)n->weights, (void *)n->act,
                     (void *)n->out, (void *)n->dA, (void *)n->dB, (void *)n->loss,
-                    (void *)n->packed, (void *)n->packed_t, (void *)n->err, (void *)n->step,
+                    (void *)n->packed, (void *)n->err, (void *)n->step,
                     (void *)n->ema_w, (void *)n->ema_weights, (void *)n->ema_table,
                     (void *)n->ema_table_bf, (void *)n->ema_packed})
         cudaFree(p);

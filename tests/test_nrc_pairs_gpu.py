@@ -55,3 +55,30 @@ def test_table_gradient(krr_lib, cuda, levels, n):
     _, dy = R.loss_and_grad(y, tgt.astype(np.float64))
     _, dX0 = R.backward(mlp, acts, dy, loss_scale=cache.cfg.loss_scale)
     assert _rel(gt, R.table_grad(grid, cs, dX0, info.n_table_entries)) < 3e-2
+
+
+@pytest.mark.parametrize("hidden", [1, 2, 5, 6, 7])
+@pytest.mark.parametrize("n", [1, 129, 20000])
+def test_layer_gradients(krr_lib, cuda, hidden, n):
+    """Every layer's gradient at each depth (seven hidden layers take the
+    CUDA-core kernels), with no full tile, a partial one and several per
+    block, against the oracle: 3e-2 of the norm, as for the trained cache."""
+    cache = NeuralRadianceCache((-1, -1, -1), (1, 1, 1), n_levels=6, log2_table_size=12, base_resolution=4,
+                                max_resolution=100, hidden_layers=hidden)
+    rng = np.random.default_rng(n)
+    cache.set_params(1, (rng.random(cache.params(1).size, dtype=np.float32) - np.float32(0.5)))
+    rec = _records(n, n)
+    tgt = _targets(rec)
+    gm, gt, loss = cache.gradients(torch.from_numpy(rec).cuda(), torch.from_numpy(tgt).cuda())
+    grid, mlp, table, info = _oracle(cache, (-1, -1, -1), (1, 1, 1))
+    X0, cs = R.encode(grid, table, rec)
+    y, acts = R.forward(mlp, X0)
+    want, dy = R.loss_and_grad(y, tgt.astype(np.float64))
+    gW, dX0 = R.backward(mlp, acts, dy, loss_scale=cache.cfg.loss_scale)
+    assert abs(loss - want) < 1e-2 * want
+    o = 0
+    for l in range(mlp.layers):
+        rows = R.WIDTH if l + 1 < mlp.layers else R.OUT_PAD
+        assert _rel(gm[o:o + rows * R.IN].reshape(rows, R.IN), gW[l]) < 3e-2, f"layer {l}"
+        o += rows * R.IN
+    assert _rel(gt, R.table_grad(grid, cs, dX0, info.n_table_entries)) < 3e-2
