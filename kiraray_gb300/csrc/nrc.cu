@@ -274,9 +274,31 @@ __global__ void k_loss(const float *__restrict__ Y, const float *__restrict__ T,
     if ((threadIdx.x & 31) == 0) atomicAdd(loss, lsum * inv);
 }
 
-// Scatter the gradient of the 32 grid features into the table gradient.
+// Advances the device step counter and stores the bias corrections.  A loss
+// that is not finite marks the cache as diverged (err[1]); a diverged cache
+// takes no further steps.  One thread, in the shadow of k_encode_bwd (the
+// double-precision powers take 9 us alone).
+struct AdamClock {
+    int64_t *step;   // null: no step is taken (gradients alone)
+    double b1, b2;
+    const float *loss;
+    uint32_t *err;
+};
+__device__ __noinline__ void adam_tick(const AdamClock &c) {
+    if (!isfinite(*c.loss)) c.err[1] = 1u;
+    if (c.err[1]) return;
+    int64_t t = *c.step + 1;
+    *c.step = t;
+    float *bc = reinterpret_cast<float *>(c.step + 1);
+    bc[0] = (float)(1.0 - pow(c.b1, (double)t));
+    bc[1] = (float)(1.0 - pow(c.b2, (double)t));
+}
+
+// Scatter the gradient of the 32 grid features into the table gradient, and
+// advance the optimiser's clock (the loss is complete by now).
 __global__ void k_encode_bwd(NrcGrid g, const float *__restrict__ in, const float *__restrict__ dX,
-                             const int32_t *d_count, int64_t cap, float *__restrict__ tgrad) {
+                             const int32_t *d_count, int64_t cap, float *__restrict__ tgrad, AdamClock clock) {
+    if (clock.step && blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) adam_tick(clock);
     int64_t n = live_count(d_count, cap);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -296,19 +318,6 @@ __global__ void k_encode_bwd(NrcGrid g, const float *__restrict__ in, const floa
 }
 
 // Adam on an FP32 master array; writes the BF16 copy and clears the gradient.
-// Advances the device step counter and stores the bias corrections.
-// A loss that is not finite marks the cache as diverged (err[1]); a diverged
-// cache takes no further steps.
-__global__ void k_adam_step(int64_t *step, double b1, double b2, const float *loss, uint32_t *err) {
-    if (!isfinite(*loss)) err[1] = 1u;
-    if (err[1]) return;
-    int64_t t = *step + 1;
-    *step = t;
-    float *bc = reinterpret_cast<float *>(step + 1);
-    bc[0] = (float)(1.0 - pow(b1, (double)t));
-    bc[1] = (float)(1.0 - pow(b2, (double)t));
-}
-
 struct AdamArgs {
     float lr, b1, b2, eps, grad_scale, bc1, bc2;
 };
@@ -318,101 +327,116 @@ struct AdamArgs {
 __device__ __forceinline__ float adam_one(const AdamArgs &a, float g, float &m, float &v, float w) {
     float gr = g * a.grad_scale;
     if (!isfinite(gr)) return w;
+    // nothing moves (and the divisions of zeros below take their slow path)
+    if (gr == 0.f && m == 0.f && v == 0.f && a.eps > 0.f) return w;
     m = a.b1 * m + (1.f - a.b1) * gr;
     v = a.b2 * v + (1.f - a.b2) * gr * gr;
     return w - a.lr * (m / a.bc1) / (sqrtf(v / a.bc2) + a.eps);
 }
 
-// Adam over n parameters (FP32 masters w, moments m and v, gradient grad which
-// is cleared, BF16 copy wb).  A thread streams two groups of four parameters
-// per step (16-byte accesses, all eight loads issued before the arithmetic):
-// the kernel is bound by HBM bandwidth, 34 bytes per parameter.
-__device__ __forceinline__ void adam4(const AdamArgs &a, float4 g, float4 &mm, float4 &vv, float4 &ww) {
-    ww.x = adam_one(a, g.x, mm.x, vv.x, ww.x);
-    ww.y = adam_one(a, g.y, mm.y, vv.y, ww.y);
-    ww.z = adam_one(a, g.z, mm.z, vv.z, ww.z);
-    ww.w = adam_one(a, g.w, mm.w, vv.w, ww.w);
-}
-
-__device__ __forceinline__ void store_bf16x4(__nv_bfloat16 *dst, int64_t i, float4 x) {
+__device__ __forceinline__ uint2 to_bf16x4(float4 x) {
     __nv_bfloat162 lo = __floats2bfloat162_rn(x.x, x.y), hi = __floats2bfloat162_rn(x.z, x.w);
-    reinterpret_cast<uint2 *>(dst)[i] =
-        make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
+    return make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
 }
 
-__device__ __forceinline__ void adam_store4(float *m, float *v, float *w, float *grad,
-                                            __nv_bfloat16 *wb, int64_t i, float4 mm, float4 vv,
-                                            float4 ww) {
-    reinterpret_cast<float4 *>(grad)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    reinterpret_cast<float4 *>(m)[i] = mm;
-    reinterpret_cast<float4 *>(v)[i] = vv;
-    reinterpret_cast<float4 *>(w)[i] = ww;
-    store_bf16x4(wb, i, ww);
-}
-
-// ema <- d ema + (1 - d) w, FP32 and BF16
-struct EmaArgs {
-    float *e;
-    __nv_bfloat16 *eb;
-    float d;
+// One array of parameters: FP32 masters w, moments m and v, gradient grad
+// (cleared), BF16 copy wb; ema <- d ema + (1 - d) w, FP32 and BF16, when kept.
+// packed, ema_packed: the MLP's weights in the tensor-core kernels' tiles,
+// written here (tensor cores only).
+struct AdamArray {
+    float *w, *m, *v, *grad;
+    __nv_bfloat16 *wb;
+    float *ema;
+    __nv_bfloat16 *ema_b;
+    int64_t n;
+    uint8_t *packed, *ema_packed;
+    int layers;
 };
-__device__ __forceinline__ void ema_store4(const EmaArgs &x, int64_t i, float4 ww) {
-    float4 e = reinterpret_cast<const float4 *>(x.e)[i];
-    const float c = 1.f - x.d;
-    e = make_float4(x.d * e.x + c * ww.x, x.d * e.y + c * ww.y, x.d * e.z + c * ww.z, x.d * e.w + c * ww.w);
-    reinterpret_cast<float4 *>(x.e)[i] = e;
-    store_bf16x4(x.eb, i, e);
+
+__device__ __forceinline__ bool any4(float4 a) { return a.x != 0.f || a.y != 0.f || a.z != 0.f || a.w != 0.f; }
+
+// Four parameters at 4 i, their gradient and moments loaded.
+__device__ __forceinline__ void adam_quad(const AdamArgs &a, const AdamArray &p, float ema_d, int64_t i, float4 g,
+                                          float4 m, float4 v) {
+    const bool moved = any4(g);
+    // no gradient yet and none before: the parameter stays, and so do its
+    // moments and its copies
+    const bool idle = !moved && !any4(m) && !any4(v) && a.eps > 0.f;
+    if (idle && !p.ema) return;
+    float4 w = reinterpret_cast<const float4 *>(p.w)[i];
+    if (!idle) {
+        w.x = adam_one(a, g.x, m.x, v.x, w.x);
+        w.y = adam_one(a, g.y, m.y, v.y, w.y);
+        w.z = adam_one(a, g.z, m.z, v.z, w.z);
+        w.w = adam_one(a, g.w, m.w, v.w, w.w);
+        if (moved) reinterpret_cast<float4 *>(p.grad)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        reinterpret_cast<float4 *>(p.m)[i] = m;
+        reinterpret_cast<float4 *>(p.v)[i] = v;
+        reinterpret_cast<float4 *>(p.w)[i] = w;
+        const uint2 b = to_bf16x4(w);
+        reinterpret_cast<uint2 *>(p.wb)[i] = b;
+        if (p.packed) *reinterpret_cast<uint2 *>(p.packed + nrc_packed_offset((int)(4 * i), p.layers)) = b;
+    }
+    if (p.ema) {
+        float4 e = reinterpret_cast<const float4 *>(p.ema)[i];
+        const float c = 1.f - ema_d;
+        e = make_float4(ema_d * e.x + c * w.x, ema_d * e.y + c * w.y, ema_d * e.z + c * w.z, ema_d * e.w + c * w.w);
+        reinterpret_cast<float4 *>(p.ema)[i] = e;
+        const uint2 b = to_bf16x4(e);
+        reinterpret_cast<uint2 *>(p.ema_b)[i] = b;
+        if (p.ema_packed) *reinterpret_cast<uint2 *>(p.ema_packed + nrc_packed_offset((int)(4 * i), p.layers)) = b;
+    }
 }
 
-__global__ void k_adam(float *__restrict__ w, float *__restrict__ m, float *__restrict__ v,
-                       float *__restrict__ grad, __nv_bfloat16 *__restrict__ wb, int64_t n, float lr,
-                       float b1, float b2, float eps, float grad_scale, const int64_t *__restrict__ step,
-                       const uint32_t *__restrict__ diverged, EmaArgs ema) {
+// Adam over the MLP (the first mlp_blocks blocks) and the table.  A parameter
+// that has never had a gradient costs its 12 bytes of gradient and moments,
+// any other 34 bytes; a third of a table of 2^19 entries a level has none on
+// the surfaces of a scene.  A thread has two groups of four parameters in
+// flight.  12.2M parameters, 65,536 records on GB300: 55 us; 128 us as two
+// launches that rewrote every parameter, half of it in the slow paths of
+// divisions and roots of zeros, and 4 us for a pack kernel.
+__global__ void __launch_bounds__(kThreads, 4)
+k_adam(AdamArray mlp, AdamArray table, int mlp_blocks, float lr, float b1, float b2, float eps,
+       float grad_scale, float ema_d, const int64_t *__restrict__ step, const uint32_t *__restrict__ diverged) {
+    const bool first = (int)blockIdx.x < mlp_blocks;
+    const AdamArray &p = first ? mlp : table;
+    const int64_t block = first ? blockIdx.x : blockIdx.x - mlp_blocks;
+    const int64_t stride = (int64_t)(first ? mlp_blocks : gridDim.x - mlp_blocks) * blockDim.x;
+    const int64_t t0 = block * blockDim.x + threadIdx.x;
     if (*diverged) {   // keep the parameters; drop the gradient
-        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-             i += (int64_t)gridDim.x * blockDim.x)
-            grad[i] = 0.f;
+        for (int64_t i = t0; i < p.n; i += stride) p.grad[i] = 0.f;
         return;
     }
-    AdamArgs a{lr, b1, b2, eps, grad_scale, reinterpret_cast<const float *>(step + 1)[0],
-               reinterpret_cast<const float *>(step + 1)[1]};
-    const int64_t n4 = n >> 2;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n4; i += 2 * stride) {
+    const AdamArgs a{lr, b1, b2, eps, grad_scale, reinterpret_cast<const float *>(step + 1)[0],
+                     reinterpret_cast<const float *>(step + 1)[1]};
+    const int64_t n4 = p.n >> 2;
+    for (int64_t i = t0; i < n4; i += 2 * stride) {
         const int64_t j = i + stride;
-        const bool two = j < n4;
-        float4 g0 = reinterpret_cast<const float4 *>(grad)[i];
-        float4 m0 = reinterpret_cast<const float4 *>(m)[i];
-        float4 v0 = reinterpret_cast<const float4 *>(v)[i];
-        float4 w0 = reinterpret_cast<const float4 *>(w)[i];
-        float4 g1{}, m1{}, v1{}, w1{};
-        if (two) {
-            g1 = reinterpret_cast<const float4 *>(grad)[j];
-            m1 = reinterpret_cast<const float4 *>(m)[j];
-            v1 = reinterpret_cast<const float4 *>(v)[j];
-            w1 = reinterpret_cast<const float4 *>(w)[j];
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 g0 = reinterpret_cast<const float4 *>(p.grad)[i];
+        const float4 m0 = reinterpret_cast<const float4 *>(p.m)[i];
+        const float4 v0 = reinterpret_cast<const float4 *>(p.v)[i];
+        float4 g1 = zero, m1 = zero, v1 = zero;
+        if (j < n4) {
+            g1 = reinterpret_cast<const float4 *>(p.grad)[j];
+            m1 = reinterpret_cast<const float4 *>(p.m)[j];
+            v1 = reinterpret_cast<const float4 *>(p.v)[j];
         }
-        adam4(a, g0, m0, v0, w0);
-        adam_store4(m, v, w, grad, wb, i, m0, v0, w0);
-        if (ema.e) ema_store4(ema, i, w0);
-        if (two) {
-            adam4(a, g1, m1, v1, w1);
-            adam_store4(m, v, w, grad, wb, j, m1, v1, w1);
-            if (ema.e) ema_store4(ema, j, w1);
-        }
+        adam_quad(a, p, ema_d, i, g0, m0, v0);
+        if (j < n4) adam_quad(a, p, ema_d, j, g1, m1, v1);
     }
-    for (int64_t i = 4 * n4 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-        float g = grad[i], mm = m[i], vv = v[i];
-        grad[i] = 0.f;
-        float ww = adam_one(a, g, mm, vv, w[i]);
-        m[i] = mm;
-        v[i] = vv;
-        w[i] = ww;
-        wb[i] = __float2bfloat16_rn(ww);
-        if (ema.e) {
-            const float e = ema.d * ema.e[i] + (1.f - ema.d) * ww;
-            ema.e[i] = e;
-            ema.eb[i] = __float2bfloat16_rn(e);
+    for (int64_t i = 4 * n4 + t0; i < p.n; i += stride) {
+        float g = p.grad[i], mm = p.m[i], vv = p.v[i];
+        p.grad[i] = 0.f;
+        float ww = adam_one(a, g, mm, vv, p.w[i]);
+        p.m[i] = mm;
+        p.v[i] = vv;
+        p.w[i] = ww;
+        p.wb[i] = __float2bfloat16_rn(ww);
+        if (p.ema) {
+            const float e = ema_d * p.ema[i] + (1.f - ema_d) * ww;
+            p.ema[i] = e;
+            p.ema_b[i] = __float2bfloat16_rn(e);
         }
     }
 }
@@ -520,8 +544,9 @@ int nrc_query_device(krr_nrc *n, const float *d_inputs, const int32_t *d_count, 
 
 // Loss, MLP backward and hash-grid backward of the last forward pass (its
 // activations in n->act): w_grad and table_grad receive the scaled gradients.
+// clock: the optimiser's, if a step follows.
 int backward(krr_nrc *n, const float *d_inputs, const float *d_targets, const int32_t *d_count,
-             int64_t cap, cudaStream_t s) {
+             int64_t cap, cudaStream_t s, AdamClock clock = {}) {
     const float scale = n->cfg.loss_scale;
     KRR_CUDA(cudaMemsetAsync(n->loss, 0, sizeof(float), s));
     float *dY = n->dA, *dX = n->dB;
@@ -556,7 +581,8 @@ int backward(krr_nrc *n, const float *d_inputs, const float *d_targets, const in
         }
     }
     // dY now holds the gradient of the encoded input
-    k_encode_bwd<<<grid_for(cap), kThreads, 0, s>>>(n->grid, d_inputs, dY, d_count, cap, n->table_grad);
+    k_encode_bwd<<<grid_for(cap), kThreads, 0, s>>>(n->grid, d_inputs, dY, d_count, cap, n->table_grad,
+                                                    clock);
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -586,22 +612,20 @@ int nrc_train_device(krr_nrc *n, const float *d_inputs, const float *d_targets,
                      const int32_t *d_count, int64_t cap, cudaStream_t s) {
     if (cap <= 0) return KRR_OK;
     KRR_TRY(forward(n, d_inputs, d_count, cap, s));
-    KRR_TRY(backward(n, d_inputs, d_targets, d_count, cap, s));
-    const float scale = n->cfg.loss_scale;
-    // Adam
     const krr_nrc_config &c = n->cfg;
-    k_adam_step<<<1, 1, 0, s>>>(n->step, (double)c.beta1, (double)c.beta2, n->loss, n->err);
-    const EmaArgs ew{n->ema_w, n->ema_weights, c.ema_decay}, et{n->ema_table, n->ema_table_bf, c.ema_decay};
-    k_adam<<<grid_for(n->mlp.n_params), kThreads, 0, s>>>(n->w_master, n->w_m, n->w_v, n->w_grad,
-                                                           n->weights, n->mlp.n_params, c.learning_rate,
-                                                           c.beta1, c.beta2, c.epsilon, 1.f / scale,
-                                                           n->step, n->err + 1, ew);
-    int64_t tn = (int64_t)n->n_entries * n->grid.features;
-    k_adam<<<grid_for(tn), kThreads, 0, s>>>(n->table_master, n->table_m, n->table_v, n->table_grad,
-                                             n->table, tn, c.learning_rate, c.beta1, c.beta2,
-                                             c.epsilon, 1.f / scale, n->step, n->err + 1, et);
+    KRR_TRY(backward(n, d_inputs, d_targets, d_count, cap, s,
+                     AdamClock{n->step, (double)c.beta1, (double)c.beta2, n->loss, n->err}));
+    uint8_t *packed = c.tensor_cores ? n->packed : nullptr, *ema_packed = c.tensor_cores ? n->ema_packed : nullptr;
+    const AdamArray mlp{n->w_master, n->w_m, n->w_v, n->w_grad, n->weights, n->ema_w, n->ema_weights,
+                        n->mlp.n_params, packed, ema_packed, n->mlp.layers};
+    const AdamArray table{n->table_master, n->table_m, n->table_v, n->table_grad, n->table, n->ema_table,
+                          n->ema_table_bf, (int64_t)n->n_entries * n->grid.features, nullptr, nullptr, 0};
+    const int mlp_blocks = grid_for((mlp.n + 3) / 4);
+    k_adam<<<mlp_blocks + grid_for((table.n + 7) / 8), kThreads, 0, s>>>(
+        mlp, table, mlp_blocks, c.learning_rate, c.beta1, c.beta2, c.epsilon, 1.f / c.loss_scale, c.ema_decay,
+        n->step, n->err + 1);
     KRR_CUDA(cudaGetLastError());
-    return pack_weights(n, s);
+    return KRR_OK;
 }
 
 }  // namespace krr

@@ -89,6 +89,14 @@ int nrc_query_device(krr_nrc *n, const float *d_inputs, const int32_t *d_count, 
 int nrc_train_device(krr_nrc *n, const float *d_inputs, const float *d_targets,
                      const int32_t *d_count, int64_t capacity, cudaStream_t s);
 int64_t nrc_batch_size(const krr_nrc *n);
+// Byte offset of MLP parameter e (row-major [out][64] weights, layer by layer)
+// in the tensor-core kernels' canonical K-major tiles: 8 KB a layer, cores of
+// 8 rows by 16 bytes.
+__host__ __device__ inline uint32_t nrc_packed_offset(int e, int layers) {
+    const int l = e / (kNrcWidth * kNrcIn) < layers - 1 ? e / (kNrcWidth * kNrcIn) : layers - 1;
+    const uint32_t local = (uint32_t)(e - l * kNrcWidth * kNrcIn), r = local / kNrcIn, k = local % kNrcIn;
+    return (uint32_t)l * (kNrcWidth * kNrcIn * 2) + ((r >> 3) * 8u + (k >> 3)) * 128u + (r & 7u) * 16u + (k & 7u) * 2u;
+}
 // tcgen05 forward (nrc_tc.cu)
 size_t nrc_tc_smem_bytes(int layers);
 int nrc_pack_weights(const __nv_bfloat16 *w, const NrcMlp &mlp, uint8_t *packed, cudaStream_t s);

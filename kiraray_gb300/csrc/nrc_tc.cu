@@ -113,14 +113,8 @@ __host__ __device__ __forceinline__ uint32_t canon(uint32_t r, uint32_t k) {
 
 // Packs the BF16 weights [layer][out][64] into canonical tiles.
 __global__ void k_pack_weights(const __nv_bfloat16 *__restrict__ w, NrcMlp mlp, uint8_t *packed) {
-    int total = mlp.n_params;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-        int l = 0;
-        while (l + 1 < mlp.layers && e >= mlp.w_offset[l + 1]) ++l;
-        int local = e - mlp.w_offset[l];
-        int r = local / kNrcIn, k = local % kNrcIn;
-        *reinterpret_cast<__nv_bfloat16 *>(packed + (size_t)l * kLayerBytes + canon(r, k)) = w[e];
-    }
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < mlp.n_params; e += gridDim.x * blockDim.x)
+        *reinterpret_cast<__nv_bfloat16 *>(packed + nrc_packed_offset(e, mlp.layers)) = w[e];
 }
 
 // Hash-grid encoding of 16 query rows by one warp, two lanes per row: lane p

@@ -82,3 +82,48 @@ def test_layer_gradients(krr_lib, cuda, hidden, n):
         assert _rel(gm[o:o + rows * R.IN].reshape(rows, R.IN), gW[l]) < 3e-2, f"layer {l}"
         o += rows * R.IN
     assert _rel(gt, R.table_grad(grid, cs, dX0, info.n_table_entries)) < 3e-2
+
+
+@pytest.mark.parametrize("levels,hidden,ema", [(1, 1, 0.0), (5, 3, 0.75), (16, 7, 0.0)])
+def test_adam_steps(krr_lib, cuda, levels, hidden, ema):
+    """Four steps on alternating batches against Adam in 64 bits on the
+    gradients that the cache reports: parameters without a gradient in a
+    step, or in any, among them.  A gradient carries the noise of FP32 atomics
+    (1e-6 of the largest), so only those above 1e-3 of the largest, or exactly
+    zero, in every step are compared: 1e-3 of the gradient's relative error,
+    doubled by m / sqrt(v), bounds a step's error by 2e-3 learning rates."""
+    cache = NeuralRadianceCache((-1, -1, -1), (1, 1, 1), n_levels=levels, log2_table_size=10, base_resolution=4,
+                                max_resolution=60, hidden_layers=hidden, epsilon=1e-12, ema_decay=ema)
+    lr, b1, b2 = cache.cfg.learning_rate, cache.cfg.beta1, cache.cfg.beta2
+    first = [cache.params(k).astype(np.float64) for k in (0, 1)]
+    w = [x.copy() for x in first]
+    m = [np.zeros_like(x) for x in first]
+    v = [np.zeros_like(x) for x in first]
+    sure = [np.ones(x.shape, bool) for x in first]
+    idle = [np.ones(x.shape, bool) for x in first]
+    for s in range(4):
+        rec = _records(300, 10 + s % 2)
+        if s % 2:
+            rec[:, :3] *= 0.3
+        r, t = torch.from_numpy(rec).cuda(), torch.from_numpy(_targets(rec)).cuda()
+        grads = cache.gradients(r, t)[:2]
+        cache.train_step(r, t)
+        for k in (0, 1):
+            g = grads[k].astype(np.float64).reshape(-1)
+            sure[k] &= (g == 0) | (np.abs(g) > 1e-3 * np.abs(g).max())
+            idle[k] &= g == 0
+            m[k] = b1 * m[k] + (1 - b1) * g
+            v[k] = b2 * v[k] + (1 - b2) * g * g
+            w[k] -= lr * (m[k] / (1 - b1 ** (s + 1))) / (np.sqrt(v[k] / (1 - b2 ** (s + 1))) + 1e-12)
+    for k in (0, 1):
+        got = cache.params(k).astype(np.float64)
+        assert sure[k].sum() > 50
+        assert np.abs(got - w[k])[sure[k]].max() <= 4 * 2e-3 * lr
+        assert np.array_equal(got[idle[k]], first[k][idle[k]])
+    # the copies that the kernels read are those of the masters
+    q = torch.from_numpy(_records(400, 3)).cuda()
+    other = NeuralRadianceCache((-1, -1, -1), (1, 1, 1), n_levels=levels, log2_table_size=10, base_resolution=4,
+                                max_resolution=60, hidden_layers=hidden)
+    for k in (0, 1):
+        other.set_params(k, cache.params(k + 2 if ema else k))
+    assert np.array_equal(cache.query(q).cpu().numpy(), other.query(q).cpu().numpy())
