@@ -1153,6 +1153,59 @@ __global__ void k_work_order(Queue q, const uint8_t *__restrict__ classes, int32
     }
 }
 
+// The walk of sampleMediumInteraction from o along dir up to tmax: queues the
+// scattering event, if one happens, and returns whether it did; thp, pu and
+// pl leave with the walk's factors (thp 0: absorbed, or given up).
+template <typename S>
+__device__ __forceinline__ bool delta_track(const DevScene &s, const DevMedium &m, V3 o, V3 dir, float tmax, Pcg &rng,
+                                            int ch, V3 &thp, S &pu, S &pl, int32_t medium, uint32_t depth,
+                                            uint32_t pixel, float time, const Queue &mscat, uint32_t *err) {
+    bool scattered = false, aborted;
+    const S T_maj = sample_t_maj<S>(m, o, dir, tmax, rng, ch, s.max_null_collisions, err, aborted,
+        [&](V3 p, const MediumProps<S> &mp, S sigma_maj, S Tm) -> bool {
+            float p_absorb = get(mp.sigma_a, ch) / get(sigma_maj, ch);
+            float p_scatter = get(mp.sigma_s, ch) / get(sigma_maj, ch);
+            float p_null = fmaxf(0.f, 1.f - p_absorb - p_scatter);
+            int mode = sample_discrete3(p_absorb, p_scatter, p_null, rng.get1d());
+            if (mode == 0) {
+                thp = v3(0.f);
+                return false;
+            }
+            if (mode == 1) {
+                const S q = over_channel(Tm * mp.sigma_s, ch);
+                thp *= q;
+                pu *= q;
+                if (any(thp) && any(pu)) {
+                    int j = push_slot(mscat.count, mscat.cap, err);
+                    if (j >= 0) {
+                        mscat.at(0, j) = f4(p, ibits(medium));
+                        mscat.at(1, j) = f4(-dir, fbits(depth));
+                        mscat.at(2, j) = f4(thp, fbits(pixel));
+                        mscat.at(3, j) = f4(v3(1.f) * pu, time);
+                    }
+                }
+                scattered = true;
+                return false;
+            }
+            const S sigma_n = vmax0(sigma_maj - mp.sigma_a - mp.sigma_s);
+            const S w = Tm * sigma_n, qn = over_channel(w, ch);
+            const float pr = get(w, ch);
+            thp *= qn;
+            if (pr == 0) thp = v3(0.f);
+            pu *= qn;
+            pl *= Tm * sigma_maj / pr;
+            return any(thp) && any(pu);
+        });
+    if (aborted) thp = v3(0.f);
+    if (!scattered && any(thp)) {
+        const S r = over_channel(T_maj, ch);
+        thp *= r;
+        pu *= r;
+        pl *= r;
+    }
+    return scattered;
+}
+
 // sampleMediumInteraction, medium.cpp:13-103 (the medium has no emission).
 // Three blocks of 256 per SM (at most 80 registers): the tracking loops are
 // latency-bound, and the extra warps outweigh a few spilled registers.
@@ -1177,52 +1230,16 @@ k_medium_sample(DevScene s, Queue msq, Queue next, Queue miss, Queue hitl, Queue
         Pcg rng = load_rng(ps, pixel);
         int ch = main_index(ps.L[pixel].w);
         const DevMedium &m = s.media[medium];
-        bool scattered = false;
-        bool aborted;
-        V3 T_maj = sample_t_maj(m, o, dir, tmax_hit, rng, ch, s.max_null_collisions, err, aborted,
-            [&](V3 p, const MediumProps &mp, V3 sigma_maj, V3 Tm) -> bool {
-                float p_absorb = get(mp.sigma_a, ch) / get(sigma_maj, ch);
-                float p_scatter = get(mp.sigma_s, ch) / get(sigma_maj, ch);
-                float p_null = fmaxf(0.f, 1.f - p_absorb - p_scatter);
-                int mode = sample_discrete3(p_absorb, p_scatter, p_null, rng.get1d());
-                if (mode == 0) {
-                    thp = v3(0.f);
-                    return false;
-                }
-                if (mode == 1) {
-                    float pr = get(Tm, ch) * get(mp.sigma_s, ch);
-                    V3 q = div_g(Tm * mp.sigma_s, pr);
-                    thp *= q;
-                    pu *= q;
-                    if (any(thp) && any(pu)) {
-                        int j = push_slot(mscat.count, mscat.cap, err);
-                        if (j >= 0) {
-                            mscat.at(0, j) = f4(p, ibits(medium));
-                            mscat.at(1, j) = f4(-dir, fbits(depth));
-                            mscat.at(2, j) = f4(thp, fbits(pixel));
-                            mscat.at(3, j) = f4(pu, time);
-                        }
-                    }
-                    scattered = true;
-                    return false;
-                }
-                V3 sigma_n = vmax(sigma_maj - mp.sigma_a - mp.sigma_s, v3(0.f));
-                float pr = get(Tm, ch) * get(sigma_n, ch);
-                V3 qn = div_g(Tm * sigma_n, pr);
-                thp *= qn;
-                if (pr == 0) thp = v3(0.f);
-                pu *= qn;
-                pl *= div_g(Tm * sigma_maj, pr);
-                return any(thp) && any(pu);
-            });
-        if (aborted) thp = v3(0.f);
-        store_rng(ps, pixel, rng);
-        if (!scattered && any(thp)) {
-            V3 r = div_g(T_maj, get(T_maj, ch));
-            thp *= r;
-            pu *= r;
-            pl *= r;
+        bool scattered;
+        if (grey(m) && grey(pu) && grey(pl)) {
+            float u1 = pu.x, l1 = pl.x;
+            scattered = delta_track(s, m, o, dir, tmax_hit, rng, ch, thp, u1, l1, medium, depth, pixel, time, mscat, err);
+            pu = v3(u1);
+            pl = v3(l1);
+        } else {
+            scattered = delta_track(s, m, o, dir, tmax_hit, rng, ch, thp, pu, pl, medium, depth, pixel, time, mscat, err);
         }
+        store_rng(ps, pixel, rng);
         if (scattered || !any(thp) || !any(pu) || (int)depth == part_of(s, pixel).max_depth) continue;
         if (isinf(tmax_hit)) {
             int j = push_slot(miss.count, miss.cap, err);
@@ -1347,6 +1364,34 @@ __global__ void k_medium_scatter(DevScene s, Queue mscat, Queue next, Queue shad
     }
 }
 
+// The walk of traceTransmittance through one medium, from o along d up to
+// t_end: T_ray, pu and pl leave with the walk's factors.
+template <typename S>
+__device__ __forceinline__ void ratio_track(const DevScene &s, const DevMedium &m, V3 o, V3 d, float t_end, Pcg &rng,
+                                            int ch, S &T_ray, S &pu, S &pl, uint32_t *err) {
+    bool aborted;
+    const S T_maj = sample_t_maj<S>(m, o, d, t_end, rng, ch, s.max_null_collisions, err, aborted,
+        [&](V3, const MediumProps<S> &mp, S sigma_maj, S Tm) -> bool {
+            const S sigma_n = vmax0(sigma_maj - mp.sigma_a - mp.sigma_s);
+            const S wm = Tm * sigma_maj;
+            const S qn = Tm * sigma_n / get(wm, ch);
+            T_ray *= qn;
+            pl *= over_channel(wm, ch);
+            pu *= qn;
+            const S Tr = T_ray / mean(pu + pl);
+            if (max_coeff(Tr) < 0.05f) {
+                if (rng.get1d() < 0.75f) T_ray = S{};
+                else T_ray /= 0.25f;
+            }
+            return any(T_ray);
+        });
+    if (aborted) T_ray = S{};
+    const S r = over_channel(T_maj, ch);
+    T_ray *= r;
+    pu *= r;
+    pl *= r;
+}
+
 // traceTransmittance (wavefront.h:80-139) for every shadow ray when media
 // are enabled: closest hits through null-material interfaces with ratio
 // tracking inside media.
@@ -1400,28 +1445,16 @@ k_shadow_tr(DevScene s, const float4 *__restrict__ nodes, const float4 *__restri
             }
             if (medium >= 0) {
                 float t_end = visible ? tmax : length(sf.p - o) / length(d);
-                bool aborted;
-                V3 T_maj = sample_t_maj(s.media[medium], o, d, t_end, rng, ch, s.max_null_collisions,
-                                        err, aborted,
-                    [&](V3, const MediumProps &mp, V3 sigma_maj, V3 Tm) -> bool {
-                        V3 sigma_n = vmax(sigma_maj - mp.sigma_a - mp.sigma_s, v3(0.f));
-                        float pr = get(Tm, ch) * get(sigma_maj, ch);
-                        V3 qn = div_g(Tm * sigma_n, pr);
-                        T_ray *= qn;
-                        pl *= div_g(Tm * sigma_maj, pr);
-                        pu *= qn;
-                        V3 Tr = div_g(T_ray, mean(pu + pl));
-                        if (max_coeff(Tr) < 0.05f) {
-                            if (rng.get1d() < 0.75f) T_ray = v3(0.f);
-                            else T_ray /= 0.25f;
-                        }
-                        return any(T_ray);
-                    });
-                if (aborted) T_ray = v3(0.f);
-                V3 r = div_g(T_maj, get(T_maj, ch));
-                T_ray *= r;
-                pu *= r;
-                pl *= r;
+                const DevMedium &m = s.media[medium];
+                if (grey(m) && grey(T_ray) && grey(pu) && grey(pl)) {
+                    float T1 = T_ray.x, u1 = pu.x, l1 = pl.x;
+                    ratio_track(s, m, o, d, t_end, rng, ch, T1, u1, l1, err);
+                    T_ray = v3(T1);
+                    pu = v3(u1);
+                    pl = v3(l1);
+                } else {
+                    ratio_track(s, m, o, d, t_end, rng, ch, T_ray, pu, pl, err);
+                }
             }
             if (visible || is_zero(T_ray)) break;
             // Interaction::spawnRayTo(pLight) from the null surface
