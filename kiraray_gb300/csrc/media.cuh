@@ -73,11 +73,11 @@ __device__ __forceinline__ float density_at(const DevMedium &m, V3 p) {
     float ix = floorf(fx), iy = floorf(fy), iz = floorf(fz);
     float u = fx - ix, v = fy - iy, w = fz - iz;
     int x0 = (int)ix, y0 = (int)iy, z0 = (int)iz;
-    // the octet of corner (x0 + sx, y0 + sy, z0 + sz): sx = 1 when x0 = -1
-    // (column -1 lies outside, column 0 is the octet's first), likewise sy, sz
-    const int sx = x0 == -1 ? 1 : 0, sy = y0 == -1 ? 1 : 0, sz = z0 == -1 ? 1 : 0;
-    float o[2][2][2] = {{{0.f, 0.f}, {0.f, 0.f}}, {{0.f, 0.f}, {0.f, 0.f}}};   // o[i][j][k]: +i x, +j y, +k z
+    float c[2][2][2] = {};   // c[i][j][k]: +i x, +j y, +k z
     if (x0 >= -1 && x0 < m.nx && y0 >= -1 && y0 < m.ny && z0 >= -1 && z0 < m.nz) {
+        // the octet of corner (x0 + sx, y0 + sy, z0 + sz): sx = 1 when x0 = -1
+        // (column -1 lies outside, column 0 is the octet's first), likewise sy, sz
+        const int sx = x0 == -1 ? 1 : 0, sy = y0 == -1 ? 1 : 0, sz = z0 == -1 ? 1 : 0;
         const uint4 q = __ldg(reinterpret_cast<const uint4 *>(m.density) +
                               ((size_t)(z0 + sz) * m.ny + (y0 + sy)) * m.nx + (x0 + sx));
         const uint32_t wd[4] = {q.x, q.y, q.z, q.w};   // word 2k + j: (x, x+1) at +j y, +k z
@@ -85,18 +85,30 @@ __device__ __forceinline__ float density_at(const DevMedium &m, V3 p) {
         for (int k = 0; k < 2; ++k)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                o[0][j][k] = half_to_float((uint16_t)(wd[2 * k + j] & 0xffffu));
-                o[1][j][k] = half_to_float((uint16_t)(wd[2 * k + j] >> 16));
+                c[0][j][k] = half_to_float((uint16_t)(wd[2 * k + j] & 0xffffu));
+                c[1][j][k] = half_to_float((uint16_t)(wd[2 * k + j] >> 16));
             }
+        // below the first voxel of an axis: shifted, zeros outside.  A branch
+        // that next to no lookup takes (1024x1024 volume frame 6.09 ms, 6.19 ms
+        // with eight selects in each lookup)
+        if (sx | sy | sz) {
+            if (sx)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) { c[1][j][k] = c[0][j][k]; c[0][j][k] = 0.f; }
+            if (sy)
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) { c[i][1][k] = c[i][0][k]; c[i][0][k] = 0.f; }
+            if (sz)
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) { c[i][j][1] = c[i][j][0]; c[i][j][0] = 0.f; }
+        }
     }
-    float c[2][2][2];
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b)
-#pragma unroll
-            for (int e = 0; e < 2; ++e)
-                c[a][b][e] = (a >= sx && b >= sy && e >= sz) ? o[a - sx][b - sy][e - sz] : 0.f;
     auto lerp = [](float a, float b, float t) { return a + t * (b - a); };
     return lerp(lerp(lerp(c[0][0][0], c[0][0][1], w), lerp(c[0][1][0], c[0][1][1], w), v),
                 lerp(lerp(c[1][0][0], c[1][0][1], w), lerp(c[1][1][0], c[1][1][1], w), v), u);
