@@ -182,7 +182,7 @@ struct Ggx {
         return Ggx{fmaxf(1e-3f, alphax), fmaxf(1e-3f, alphay)};
     }
     KRR_D bool is_delta() const { return fmaxf(ax, ay) <= 1e-3f; }
-    KRR_D float lambda(V3 w) const {
+    __device__ __noinline__ float lambda(V3 w) const {
         float abs_tan = fabsf(tan_theta(w));
         if (isinf(abs_tan)) return 0.f;
         float c = cos_phi(w), s = sin_phi(w);
@@ -192,7 +192,7 @@ struct Ggx {
     }
     KRR_D float g1(V3 w) const { return 1 / (1 + lambda(w)); }
     KRR_D float g(V3 wo, V3 wi) const { return 1 / (1 + lambda(wo) + lambda(wi)); }
-    KRR_D float d(V3 wh) const {
+    __device__ __noinline__ float d(V3 wh) const {
         float t2 = tan2_theta(wh);
         if (isinf(t2)) return 0.f;
         float c2 = cos2_theta(wh);
@@ -293,7 +293,9 @@ KRR_D Cx cx_sqrt(Cx z) {
     return {fabsf(t2), copysignf(t1, z.im)};
 }
 
-KRR_D float fr_complex(float cos_i, Cx eta) {
+// A function of its own, as Ggx::lambda and Ggx::d: a path's shading uses each
+// several times, and its time is to a good part that of fetching instructions.
+static __device__ __noinline__ float fr_complex(float cos_i, Cx eta) {
     cos_i = fminf(fmaxf(cos_i, 0.f), 1.f);
     float sin2_i = 1 - cos_i * cos_i;
     Cx sin2_t = cx_div(Cx{sin2_i, 0}, cx_mul(eta, eta));
@@ -377,11 +379,18 @@ struct Bsdf {
         return b;
     }
 
-    // f(), TransportMode::Radiance
-    KRR_D V3 f(V3 wo, V3 wi) const {
+    // Diffuse f() and pdf() (diffuse.h:33-49).
+    KRR_D V3 diffuse_f(V3 wo, V3 wi) const { return same_hemisphere(wo, wi) ? color * kInvPi : v3(0.f); }
+    KRR_D float diffuse_pdf(V3 wo, V3 wi) const { return same_hemisphere(wo, wi) ? fabsf(wi.z) * kInvPi : 0.f; }
+
+    // f() (TransportMode::Radiance), and pdf() wherever f is not 0.  Both of
+    // a rough BSDF need the microfacet normal, its density (the same for wm
+    // and -wm: it holds squares alone) and the masking of wo: computed once.
+    KRR_D V3 eval(V3 wo, V3 wi, float &pdf) const {
+        pdf = 0.f;
         if (type == MAT_DIFFUSE) {
-            if (!same_hemisphere(wo, wi)) return v3(0.f);
-            return color * kInvPi;
+            pdf = diffuse_pdf(wo, wi);
+            return diffuse_f(wo, wi);
         }
         if (type == MAT_CONDUCTOR) {
             if (!same_hemisphere(wo, wi)) return v3(0.f);
@@ -391,8 +400,10 @@ struct Bsdf {
             V3 wm = wi + wo;
             if (length_sq(wm) == 0) return v3(0.f);
             wm = normalize(wm);
-            V3 F = fr_complex3(fabsf(dot(wo, wm)), eta3, k3);
-            return dist.d(wm) * F * dist.g(wo, wi) / (4 * ci * co);
+            const float owm = fabsf(dot(wo, wm)), D = dist.d(wm), lo = dist.lambda(wo);
+            V3 F = fr_complex3(owm, eta3, k3);
+            pdf = D * (1 / (1 + lo)) * owm / co / (4 * owm);
+            return D * F * (1 / (1 + lo + dist.lambda(wi))) / (4 * ci * co);
         }
         if (type == MAT_DIELECTRIC) {
             if (eta == 1 || dist.is_delta()) return v3(0.f);
@@ -402,54 +413,29 @@ struct Bsdf {
             if (!refl) etap = co > 0 ? eta : (1 / eta);
             V3 wm = wi * etap + wo;
             if (ci == 0 || co == 0 || !any(wm)) return v3(0.f);
+            const bool tiny = length_sq(wm) == 0;
             wm = face_forward(normalize(wm), V3{0, 0, 1});
-            if (dot(wm, wi) * ci < 0 || dot(wm, wo) * co < 0) return v3(0.f);
-            float F = fr_dielectric(copysignf(dot(wo, wm), wo.z), eta);
+            const float om = dot(wo, wm), im = dot(wi, wm);
+            if (im * ci < 0 || om * co < 0) return v3(0.f);
+            const float D = dist.d(wm), lo = dist.lambda(wo), G = 1 / (1 + lo + dist.lambda(wi));
+            const float pm = D * (1 / (1 + lo)) * fabsf(om) / abs_cos_theta(wo);   // of wm
+            float F = fr_dielectric(copysignf(om, wo.z), eta);
             V3 R = color * F, T = color * (1 - F);
-            if (refl) return dist.d(wm) * dist.g(wo, wi) * R / fabsf(4 * ci * co);
-            float dwi = dot(wi, wm) + dot(wo, wm) / etap;
+            float Fz = fr_dielectric(wo.z, eta);   // the lobes' shares in pdf()
+            V3 Rz = color * Fz, Tz = color * (1 - Fz);
+            float pr = mean(Rz), pt = mean(Tz);
+            const bool none = tiny || (pr == 0 && pt == 0);
+            if (refl) {
+                if (!none) pdf = pm / (4 * fabsf(om)) * pr / (pr + pt);
+                return D * G * R / fabsf(4 * ci * co);
+            }
+            float dwi = im + om / etap;
+            if (!none) pdf = pm * (fabsf(im) / (dwi * dwi)) * pt / (pr + pt);
             float denom = dwi * dwi * ci * co;
-            V3 ft = T * dist.d(wm) * dist.g(wo, wi) * fabsf(dot(wi, wm) * dot(wo, wm) / denom);
-            ft = ft / (etap * etap);
-            return ft;
+            V3 ft = T * D * G * fabsf(im * om / denom);
+            return ft / (etap * etap);
         }
         return v3(0.f);
-    }
-
-    KRR_D float pdf(V3 wo, V3 wi) const {
-        if (type == MAT_DIFFUSE) {
-            if (!same_hemisphere(wo, wi)) return 0.f;
-            return fabsf(wi.z) * kInvPi;
-        }
-        if (type == MAT_CONDUCTOR) {
-            if (!same_hemisphere(wo, wi)) return 0.f;
-            if (dist.is_delta()) return 0.f;
-            V3 wm = wo + wi;
-            if (is_zero(wm)) return 0.f;
-            wm = face_forward(normalize(wm), V3{0, 0, 1});
-            return dist.pdf(wo, wm) / (4 * fabsf(dot(wo, wm)));
-        }
-        if (type == MAT_DIELECTRIC) {
-            if (eta == 1 || dist.is_delta()) return 0.f;
-            float co = wo.z, ci = wi.z;
-            bool refl = ci * co > 0;
-            float etap = 1;
-            if (!refl) etap = co > 0 ? eta : (1 / eta);
-            V3 wm = wi * etap + wo;
-            if (ci == 0 || co == 0 || length_sq(wm) == 0) return 0.f;
-            wm = face_forward(normalize(wm), V3{0, 0, 1});
-            if (dot(wm, wi) * ci < 0 || dot(wm, wo) * co < 0) return 0.f;
-            float F = fr_dielectric(wo.z, eta);
-            V3 R = color * F, T = color * (1 - F);
-            float pr = mean(R), pt = mean(T);
-            if (pr == 0 && pt == 0) return 0.f;
-            if (refl) return dist.pdf(wo, wm) / (4 * fabsf(dot(wo, wm))) * pr / (pr + pt);
-            float dwi = dot(wi, wm) + dot(wo, wm) / etap;
-            float denom = dwi * dwi;
-            float dwm_dwi = fabsf(dot(wi, wm)) / denom;
-            return dist.pdf(wo, wm) * dwm_dwi * pt / (pr + pt);
-        }
-        return 0.f;
     }
 
     template <typename Draw>
@@ -461,8 +447,8 @@ struct Bsdf {
             V3 wi = cosine_sample_hemisphere(u0, u1);
             wi.z = wi.z * wo.z > 0 ? wi.z : -wi.z;   // ToSameHemisphere
             s.wi = wi;
-            s.f = f(wo, wi);
-            s.pdf = pdf(wo, wi);
+            s.f = diffuse_f(wo, wi);
+            s.pdf = diffuse_pdf(wo, wi);
             s.flags = BSDF_DIFFUSE_REFLECTION;
             return s;
         }

@@ -938,11 +938,12 @@ __global__ void k_handle_miss(DevScene s, Queue miss, PixelState ps, int nee) {
 // When `tracked` has a counter (a pass of several scenes, some with media),
 // the shadow ray of a scene with media goes straight to the transmittance
 // tracker's queue and `shadow` keeps only the rays that an any-hit test
-// decides.
+// decides.  `light` and `bounce`: whether to do the light sample (shadow ray)
+// and the BSDF sample (next ray, and the sampler's new state).
 __device__ __forceinline__ void scatter_item(const DevScene &s, const Queue &scat, int i, Pcg rng,
                                              const Queue &next, const Queue &shadow_q,
                                              const Queue &tracked, const PixelState &ps, int nee,
-                                             float rr, uint32_t *err) {
+                                             float rr, bool light, bool bounce, uint32_t *err) {
     float4 c0 = scat.at(0, i), c1 = scat.at(1, i), c2 = scat.at(2, i), c3 = scat.at(3, i);
     float4 c4 = scat.at(4, i), c5 = scat.at(5, i), c6 = scat.at(6, i), c7 = scat.at(7, i);
     uint32_t pixel = ubits(c2.w), depth = ubits(c1.w);
@@ -964,36 +965,39 @@ __device__ __forceinline__ void scatter_item(const DevScene &s, const Queue &sca
     const Queue &shadow = (tracked.count && P.has_media) ? tracked : shadow_q;
     if (nee && (bsdf_type & BSDF_SMOOTH) && P.n_lights > 0) {
         float ul = rng.get1d();
-        uint32_t lid = (uint32_t)(ul * (float)P.n_lights);
-        float sel_pdf = 1.f / (float)P.n_lights;
         float u0 = rng.get1d(), u1 = rng.get1d();
-        LightSample ls = sample_li(s, s.lights[P.light_begin + lid], u0, u1, p);
-        // spawnRayTo(Interaction), raytracing.h:151-160
-        V3 to = offset_ray_origin(ls.p, ls.n, p - ls.p);
-        V3 po = offset_ray_origin(p, nrm, to - p);
-        V3 d = to - po;
-        V3 wi_world = normalize(d);
-        V3 wi_local = to_local(wi_world);
-        float light_pdf = sel_pdf * ls.pdf;
-        V3 fv = bsdf.f(wo_local, wi_local);
-        float bsdf_pdf = bsdf.pdf(wo_local, wi_local);
-        if (light_pdf > 0 && any(fv)) {
-            V3 Ld = ls.L * thp * fv * fabsf(wi_local.z);
-            if (any(Ld)) {
-                // with a tracker queue the lanes of a warp may push to two queues
-                int j = tracked.count ? push_slot_grouped(shadow.count, shadow.cap, err)
-                                      : push_slot(shadow.count, shadow.cap, err);
-                if (j >= 0) {
-                    int32_t med = medium_towards(mi, mo, ray_medium, nrm, d);
-                    shadow.at(0, j) = f4(po, 0.f);
-                    shadow.at(1, j) = f4(d, 1.f);
-                    shadow.at(2, j) = f4(Ld, fbits(pixel));
-                    shadow.at(3, j) = f4(pu * bsdf_pdf, ibits(med));
-                    shadow.at(4, j) = f4(pu * light_pdf, time);
+        if (light) {
+            uint32_t lid = (uint32_t)(ul * (float)P.n_lights);
+            float sel_pdf = 1.f / (float)P.n_lights;
+            LightSample ls = sample_li(s, s.lights[P.light_begin + lid], u0, u1, p);
+            // spawnRayTo(Interaction), raytracing.h:151-160
+            V3 to = offset_ray_origin(ls.p, ls.n, p - ls.p);
+            V3 po = offset_ray_origin(p, nrm, to - p);
+            V3 d = to - po;
+            V3 wi_world = normalize(d);
+            V3 wi_local = to_local(wi_world);
+            float light_pdf = sel_pdf * ls.pdf;
+            float bsdf_pdf;
+            V3 fv = bsdf.eval(wo_local, wi_local, bsdf_pdf);
+            if (light_pdf > 0 && any(fv)) {
+                V3 Ld = ls.L * thp * fv * fabsf(wi_local.z);
+                if (any(Ld)) {
+                    // with a tracker queue the lanes of a warp may push to two queues
+                    int j = tracked.count ? push_slot_grouped(shadow.count, shadow.cap, err)
+                                          : push_slot(shadow.count, shadow.cap, err);
+                    if (j >= 0) {
+                        int32_t med = medium_towards(mi, mo, ray_medium, nrm, d);
+                        shadow.at(0, j) = f4(po, 0.f);
+                        shadow.at(1, j) = f4(d, 1.f);
+                        shadow.at(2, j) = f4(Ld, fbits(pixel));
+                        shadow.at(3, j) = f4(pu * bsdf_pdf, ibits(med));
+                        shadow.at(4, j) = f4(pu * light_pdf, time);
+                    }
                 }
             }
         }
     }
+    if (!bounce) return;
     BsdfSample bs = bsdf.sample(wo_local, [&]() { return rng.get1d(); });
     store_rng(ps, pixel, rng);
     if (bs.pdf != 0 && any(bs.f)) {
@@ -1052,20 +1056,51 @@ __global__ void k_scatter_classify(DevScene s, Queue scat, PixelState ps, float 
 
 // Three blocks per SM (80 registers, 104 bytes spilled): 0.8 % faster per
 // 1080p frame than four blocks at 64 registers (236 bytes spilled).
+//
+// A launch of few items lasts as long as one item's chain of instructions,
+// some thousands that nobody has fetched before, and a dozen dependent loads:
+// 40 us.  While the resident blocks (`resident`) have two threads for each
+// item, one warp of a pair does its 32 items' light samples and the other
+// their BSDF samples; both take the sampler's state before the second stores
+// the new one.  With that, Bsdf::eval and the Fresnel and microfacet terms as
+// functions of their own (fewer instructions to fetch) on GB300: 27-30 us,
+// frames at 241x135 1,012 and 934 us, at 1920x1080 4.91 and 4.76 ms.
 __global__ void __launch_bounds__(kThreads, 3)
 k_scatter_process(DevScene s, Queue scat, const int32_t *__restrict__ lists,
                   const int32_t *__restrict__ counts, Queue next, Queue shadow, Queue tracked,
-                  PixelState ps, int nee, float rr, uint32_t *err) {
+                  PixelState ps, int nee, float rr, int resident, uint32_t *err) {
     const int cap = scat.cap;
     const int c0 = counts[0], c01 = c0 + counts[1], c012 = c01 + counts[2], total = c012 + counts[3];
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-        const int i = g < c0 ? lists[g]
-                    : g < c01 ? lists[cap - 1 - (g - c0)]
-                    : g < c012 ? lists[cap + (g - c01)]
-                    : lists[2 * (size_t)cap - 1 - (g - c012)];
-        Pcg rng = load_rng(ps, ubits(scat.at(2, i).w));
-        rng.get1d();   // the roulette draw taken by k_scatter_classify
-        scatter_item(s, scat, i, rng, next, shadow, tracked, ps, nee, rr, err);
+    auto item = [&](int g) {
+        return g < c0 ? lists[g]
+             : g < c01 ? lists[cap - 1 - (g - c0)]
+             : g < c012 ? lists[cap + (g - c01)]
+             : lists[2 * (size_t)cap - 1 - (g - c012)];
+    };
+    const int first = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+    const int pairs = (total + 31) / 32;
+    const bool split = nee && pairs <= resident * (int)blockDim.x / 64;
+    bool light = true, bounce = true;
+    for (int g0 = first; g0 < (split ? threads : total); g0 += threads) {
+        int g = g0;
+        if (split) {
+            // both warps of a pair in one block, the pairs spread over the blocks
+            const int w = threadIdx.x >> 5;
+            g = (int)blockIdx.x < resident ? ((w >> 1) * resident + (int)blockIdx.x) * 32 + (threadIdx.x & 31) : total;
+            light = w & 1;
+            bounce = !light;
+        }
+        int i = 0;
+        Pcg rng;
+        if (g < total) {
+            i = item(g);
+            rng = load_rng(ps, ubits(scat.at(2, i).w));
+        }
+        if (split) __syncthreads();   // every light sample's state is read before one is stored
+        if (g < total) {
+            rng.get1d();   // the roulette draw taken by k_scatter_classify
+            scatter_item(s, scat, i, rng, next, shadow, tracked, ps, nee, rr, light, bounce, err);
+        }
     }
 }
 
@@ -1666,8 +1701,8 @@ __device__ __forceinline__ bool mk_bounce(const DevScene &s, const WfConst &c, c
             V3 wi_world = normalize(d);
             V3 wi_local = to_local(wi_world);
             float light_pdf = sel_pdf * ls.pdf;
-            V3 fv = bsdf.f(wo_local, wi_local);
-            float bsdf_pdf = bsdf.pdf(wo_local, wi_local);
+            float bsdf_pdf;
+            V3 fv = bsdf.eval(wo_local, wi_local, bsdf_pdf);
             if (light_pdf > 0 && any(fv)) {
                 V3 Ld = ls.L * sthp * fv * fabsf(wi_local.z);
                 if (any(Ld)) {
@@ -2865,6 +2900,15 @@ extern "C" int krr_wf_handle_miss(krr_wf *wf, void *stream) {
     return KRR_OK;
 }
 
+// Blocks of a stage kernel of which `per_sm` blocks of kThreads fit an SM: the
+// pass's, at most those that are resident at once.
+static int resident_grid(const krr_wf *wf, int per_sm) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return std::min(wf->grid, std::max(1, sms) * per_sm * kThreads / wf->block);
+}
+
 // generateScatterRays; with `to_tracker` the shadow rays of scenes with
 // media go to their own queue for k_shadow_split (split_shadows()).
 static int scatter_stage(krr_wf *wf, int depth, cudaStream_t st, bool to_tracker) {
@@ -2879,7 +2923,7 @@ static int scatter_stage(krr_wf *wf, int depth, cudaStream_t st, bool to_tracker
     k_scatter_process<<<wf->grid, wf->block, 0, st>>>(wf->scene, wf->q(Q_SCATTER), wf->scatter_lists,
                                                      wf->scatter_class_counts(), wf->q(cur ^ 1),
                                                      wf->q(Q_SHADOW), tracked, wf->ps, wf->params.nee,
-                                                     wf->params.rr, wf->err());
+                                                     wf->params.rr, resident_grid(wf, 3), wf->err());
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -3420,15 +3464,6 @@ extern "C" int krr_wf_group_launch(krr_wf_group *g, int64_t frame_index, void *s
 }
 
 namespace krr {
-// Blocks of a tracking launch: the resident ones (three of 256 threads per
-// SM), which deal the items out among themselves.
-static int tracking_grid(const krr_wf *wf) {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return std::min(wf->grid, std::max(1, sms) * 3 * kThreads / wf->block);
-}
-
 // The permutation of a tracking queue's items by work class (media work
 // order, above), in the scatter-list buffer (free during the media stages).
 static int work_order(krr_wf *wf, const Queue &q, int items, cudaStream_t st, const int32_t **order) {
@@ -3448,7 +3483,7 @@ static int work_order(krr_wf *wf, const Queue &q, int items, cudaStream_t st, co
 int launch_medium_sample(krr_wf *wf, int depth, cudaStream_t st) {
     const int32_t *order = nullptr;
     KRR_TRY(work_order(wf, wf->q(Q_MEDIUM_SAMPLE), 0, st, &order));
-    k_medium_sample<<<tracking_grid(wf), wf->block, 0, st>>>(wf->scene, wf->q(Q_MEDIUM_SAMPLE),
+    k_medium_sample<<<resident_grid(wf, 3), wf->block, 0, st>>>(wf->scene, wf->q(Q_MEDIUM_SAMPLE),
                                                     wf->q((depth & 1) ^ 1), wf->q(Q_MISS),
                                                     wf->q(Q_HIT_LIGHT), wf->q(Q_SCATTER),
                                                     wf->q(Q_MEDIUM_SCATTER), wf->ps, order,
@@ -3533,7 +3568,7 @@ int launch_shadow_tracker(krr_wf *wf, cudaStream_t st) {
     const int32_t *order = nullptr;
     KRR_TRY(work_order(wf, tracked, 1, st, &order));
 #define KRR_SHADOW_TR(F, LV)                                                                           \
-    k_shadow_tr<F, LV><<<tracking_grid(wf), wf->block, 0, st>>>(wf->scene, wf->accel.d_nodes, wf->accel.d_tris, iv, \
+    k_shadow_tr<F, LV><<<resident_grid(wf, 3), wf->block, 0, st>>>(wf->scene, wf->accel.d_nodes, wf->accel.d_tris, iv, \
                                                        tracked, wf->ps, order, wf->deal_cursor(1), wf->err(), terr)
     const bool two = wf->accel.levels == 2, f1 = wf->accel.node_format == 1;
     if (two) { if (f1) KRR_SHADOW_TR(1, 2); else KRR_SHADOW_TR(0, 2); }
