@@ -1141,6 +1141,7 @@ template <int MODE, bool STATS, int FMT>
 __global__ void __launch_bounds__(kTraceThreads, FMT != 1 ? 8 : 1)
 k_trace(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, TraceLaunch L,
         unsigned long long *stats) {
+    stream_order();
     trace_body<MODE, STATS, FMT>(nodes, tris, L, stats);
 }
 
@@ -1149,6 +1150,7 @@ k_trace(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, Trace
 template <int FMT>
 __global__ void __launch_bounds__(kTraceThreads, FMT != 1 ? 8 : 1)
 k_trace_mixed(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, TraceLaunch L) {
+    stream_order();
     trace_body<2, false, FMT>(nodes, tris, L, nullptr);
 }
 
@@ -1210,18 +1212,18 @@ static int launch_trace(const krr_accel *a, const TraceLaunch &l, cudaStream_t s
     const bool single = a->max_leaf == 1 && a->full_leaf == 1;
     if constexpr (MODE == 2) {
         if (a->node_format == 1)
-            k_trace_mixed<1><<<grid, kTraceThreads, 0, s>>>(a->d_nodes, a->d_tris, lt);
+            KRR_CUDA(launch_ordered(k_trace_mixed<1>, grid, kTraceThreads, s, a->d_nodes, a->d_tris, lt));
         else if (single)
-            k_trace_mixed<2><<<grid, kTraceThreads, 0, s>>>(a->d_nodes, a->d_tris, lt);
+            KRR_CUDA(launch_ordered(k_trace_mixed<2>, grid, kTraceThreads, s, a->d_nodes, a->d_tris, lt));
         else
-            k_trace_mixed<0><<<grid, kTraceThreads, 0, s>>>(a->d_nodes, a->d_tris, lt);
+            KRR_CUDA(launch_ordered(k_trace_mixed<0>, grid, kTraceThreads, s, a->d_nodes, a->d_tris, lt));
     } else {
         if (a->node_format == 1)
-            k_trace<MODE, STATS, 1><<<grid, kTraceThreads, 0, s>>>(a->d_nodes, a->d_tris, lt, stats);
+            KRR_CUDA(launch_ordered(k_trace<MODE, STATS, 1>, grid, kTraceThreads, s, a->d_nodes, a->d_tris, lt, stats));
         else if (single)
-            k_trace<MODE, STATS, 2><<<grid, kTraceThreads, 0, s>>>(a->d_nodes, a->d_tris, lt, stats);
+            KRR_CUDA(launch_ordered(k_trace<MODE, STATS, 2>, grid, kTraceThreads, s, a->d_nodes, a->d_tris, lt, stats));
         else
-            k_trace<MODE, STATS, 0><<<grid, kTraceThreads, 0, s>>>(a->d_nodes, a->d_tris, lt, stats);
+            KRR_CUDA(launch_ordered(k_trace<MODE, STATS, 0>, grid, kTraceThreads, s, a->d_nodes, a->d_tris, lt, stats));
     }
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;

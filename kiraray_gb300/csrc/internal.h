@@ -29,6 +29,26 @@ enum DeviceError : uint32_t {
     kErrBadInput = 1u << 3,
 };
 
+// Launches a kernel that may be brought up while the one before it on the
+// stream still runs; the kernel starts with stream_order() (kmath.cuh), which
+// waits for that one's end and its writes.  Between short dependent kernels
+// this hides the launch itself.  After anything that is not such a kernel
+// (copies, memsets, other launches) and for anything after it, the order is
+// the stream's as always.
+template <typename... P, typename... A>
+inline cudaError_t launch_ordered(void (*kernel)(P...), int grid, int block, cudaStream_t s, A &&...args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace krr
 
 #define KRR_CUDA(call)                                                              \

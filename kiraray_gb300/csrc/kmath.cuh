@@ -16,6 +16,14 @@ constexpr float kInv4Pi = 0.07957747154594766788f;
 constexpr float k2Pi = 6.28318530717958647692f;
 constexpr float kRayEps = 1e-4f;   // KRR_RAY_EPS, src/core/raytracing.h:10
 
+// First statement of a kernel that launch_ordered() starts: the kernel before
+// it on the stream has ended and its writes are visible; and the kernel after
+// it may be brought up.
+KRR_D void stream_order() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 struct V3 {
     float x, y, z;
 };

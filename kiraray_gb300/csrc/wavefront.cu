@@ -128,7 +128,9 @@ struct krr_wf {
                                    // batches, [11] ratio-tracked shadow rays, [12-15]
                                    // scatter items per material class, [16] shadow
                                    // rays of scenes with media (split routing),
-                                   // [18-21] cursors of the tracking launches
+                                   // [17] finished blocks of a
+                                   // scatter launch, [18-21] cursors of the tracking launches;
+                                   // 11-15 and 17-21 are 0 between launches
     float4 *media_shadow = nullptr;   // [kShadowCh][qcap], split routing only
     float4 *hits = nullptr;
     uint8_t *occluded = nullptr;
@@ -162,6 +164,7 @@ struct krr_wf {
     int32_t *shadow_tracked_count() const { return d_counts + 11; }
     int32_t *scatter_class_counts() const { return d_counts + 12; }
     int32_t *media_shadow_count() const { return d_counts + 16; }
+    int32_t *scatter_blocks_done() const { return d_counts + 17; }
     int32_t *deal_cursor(int k) const { return d_counts + 18 + 2 * k; }   // of a tracking launch
     uint32_t *err() const { return reinterpret_cast<uint32_t *>(d_counts + 8); }
     WfConst consts() const {
@@ -311,11 +314,12 @@ struct Deal {
         if (base >= n) return -2;
         return lane < count && base + lane < n ? base + lane : -1;
     }
-    // every warp, once, after its last take
-    __device__ void done() const {
+    // every warp, once, after its last take; the last one empties `queue`, if given
+    __device__ void done(int32_t *queue = nullptr) const {
         if ((threadIdx.x & 31) == 0 && atomicAdd(cursor + 1, 1) == warps - 1) {
             cursor[0] = 0;
             cursor[1] = 0;
+            if (queue) *queue = 0;
         }
     }
 };
@@ -589,6 +593,7 @@ __device__ __forceinline__ int64_t tile_pixel(int64_t i, int w, int h) {
 // pixel, so frames are the same in either order.
 __global__ void k_camera_rays(PixelState ps, Queue rq, const DevView *__restrict__ views,
                               const FrameConst *__restrict__ fc, int64_t p0, int64_t n, int tiled) {
+    stream_order();
     if (blockIdx.x == 0 && threadIdx.x == 0) *rq.count = (int32_t)n;
     const int nv = fc->n_views;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
@@ -623,6 +628,7 @@ __global__ void k_camera_rays(PixelState ps, Queue rq, const DevView *__restrict
 }
 
 __global__ void k_reset_queues(int32_t *counts, int cur, int all) {
+    stream_order();
     if (threadIdx.x == 0) {
         for (int k = 0; k < Q_COUNT; ++k)
             if (all || k != cur) counts[k] = 0;
@@ -719,6 +725,7 @@ __device__ __forceinline__ bool nrc_vertex(const NrcHook &h, const DevScene &s, 
 // L[pixel] += throughput x max(cache, 0)
 __global__ void k_nrc_apply(const float *__restrict__ out, const float4 *__restrict__ meta,
                             const int32_t *count, int cap, PixelState ps) {
+    stream_order();
     int n = min(*count, cap);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float4 m = meta[i];
@@ -813,6 +820,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 k_hit_process(DevScene s, Queue rq, const float4 *__restrict__ hits, Queue next, Queue miss,
               Queue hitl, Queue scat, Queue msq, int enable_medium, uint32_t *err, NrcHook hook,
               PixelState ps, int inline_lights, int nee) {
+    stream_order();
     int n = min(*rq.count, rq.cap);   // an overflowed queue holds cap items
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float4 h = hits[i];
@@ -911,6 +919,7 @@ k_hit_process(DevScene s, Queue rq, const float4 *__restrict__ hits, Queue next,
 
 // handleHit, integrator.cpp:78-90
 __global__ void k_handle_hit(DevScene s, Queue hitl, PixelState ps, int nee) {
+    stream_order();
     int n = min(*hitl.count, hitl.cap);   // an overflowed queue holds cap items
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float4 c0 = hitl.at(0, i), c1 = hitl.at(1, i), c2 = hitl.at(2, i), c3 = hitl.at(3, i);
@@ -923,6 +932,7 @@ __global__ void k_handle_hit(DevScene s, Queue hitl, PixelState ps, int nee) {
 
 // handleMiss, integrator.cpp:92-108
 __global__ void k_handle_miss(DevScene s, Queue miss, PixelState ps, int nee) {
+    stream_order();
     int n = min(*miss.count, miss.cap);   // an overflowed queue holds cap items
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float4 c1 = miss.at(1, i), c3 = miss.at(3, i), c4 = miss.at(4, i), c5 = miss.at(5, i),
@@ -1031,6 +1041,7 @@ __device__ __forceinline__ void scatter_item(const DevScene &s, const Queue &sca
 // sampler stream is its pixel's); only the order of the queue pushes changes.
 __global__ void k_scatter_classify(DevScene s, Queue scat, PixelState ps, float rr,
                                    int32_t *__restrict__ lists, int32_t *__restrict__ counts) {
+    stream_order();
     const int cap = scat.cap, n = min(*scat.count, cap);
     const int lane = threadIdx.x & 31;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1067,8 +1078,9 @@ __global__ void k_scatter_classify(DevScene s, Queue scat, PixelState ps, float 
 // frames at 241x135 1,012 and 934 us, at 1920x1080 4.91 and 4.76 ms.
 __global__ void __launch_bounds__(kThreads, 3)
 k_scatter_process(DevScene s, Queue scat, const int32_t *__restrict__ lists,
-                  const int32_t *__restrict__ counts, Queue next, Queue shadow, Queue tracked,
+                  int32_t *counts, int32_t *blocks_done, Queue next, Queue shadow, Queue tracked,
                   PixelState ps, int nee, float rr, int resident, uint32_t *err) {
+    stream_order();
     const int cap = scat.cap;
     const int c0 = counts[0], c01 = c0 + counts[1], c012 = c01 + counts[2], total = c012 + counts[3];
     auto item = [&](int g) {
@@ -1102,10 +1114,18 @@ k_scatter_process(DevScene s, Queue scat, const int32_t *__restrict__ lists,
             scatter_item(s, scat, i, rng, next, shadow, tracked, ps, nee, rr, light, bounce, err);
         }
     }
+    // the last block leaves the class counts 0 for the next launch of
+    // k_scatter_classify
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(blocks_done, 1) == (int)gridDim.x - 1) {
+        for (int k = 0; k < 4; ++k) counts[k] = 0;
+        *blocks_done = 0;
+    }
 }
 
 // Radiance of unoccluded shadow rays (__raygen__Shadow, device.cu:92-100).
 __global__ void k_shadow_resolve(Queue shadow, const uint8_t *__restrict__ occluded, PixelState ps) {
+    stream_order();
     int n = min(*shadow.count, shadow.cap);   // an overflowed queue holds cap items
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (occluded[i]) continue;
@@ -1247,6 +1267,7 @@ __device__ __forceinline__ bool delta_track(const DevScene &s, const DevMedium &
 __global__ void __launch_bounds__(kThreads, 3)
 k_medium_sample(DevScene s, Queue msq, Queue next, Queue miss, Queue hitl, Queue scat,
                 Queue mscat, PixelState ps, const int32_t *__restrict__ order, int32_t *cursor, uint32_t *err) {
+    stream_order();
     int n = min(*msq.count, msq.cap);   // an overflowed queue holds cap items
     const Deal deal(cursor);
     while (true) {
@@ -1334,6 +1355,7 @@ k_medium_sample(DevScene s, Queue msq, Queue next, Queue miss, Queue hitl, Queue
 // straight to the transmittance tracker's queue, as in scatter_item.
 __global__ void k_medium_scatter(DevScene s, Queue mscat, Queue next, Queue shadow_q, Queue tracked,
                                  PixelState ps, int nee, uint32_t *err) {
+    stream_order();
     const Queue &shadow = tracked.count ? tracked : shadow_q;
     int n = min(*mscat.count, mscat.cap);   // an overflowed queue holds cap items
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1448,6 +1470,7 @@ __global__ void __launch_bounds__(kThreads, 3)
 k_shadow_tr(DevScene s, const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
             InstancedView iv, Queue shadow, PixelState ps, const int32_t *__restrict__ order,
             int32_t *cursor, uint32_t *err, int *trace_err) {
+    stream_order();
     int n = min(*shadow.count, shadow.cap);   // an overflowed queue holds cap items
     const Deal deal(cursor);
     while (true) {
@@ -1508,7 +1531,7 @@ k_shadow_tr(DevScene s, const float4 *__restrict__ nodes, const float4 *__restri
         if (any(T_ray))
             add_radiance(ps, pixel, f3(c2) * T_ray / mean(f3(c3) * pu + f3(c4) * pl));
     }
-    deal.done();
+    deal.done(shadow.count);
 }
 
 // First pass of the transmittance shadow stage.  A shadow ray that starts
@@ -1527,6 +1550,7 @@ template <int FMT, int LEVELS>
 __global__ void k_shadow_split(DevScene s, const float4 *__restrict__ nodes,
                                const float4 *__restrict__ tris, InstancedView iv, Queue shadow,
                                Queue tracked, PixelState ps, uint32_t *err, int *trace_err) {
+    stream_order();
     int n = min(*shadow.count, shadow.cap);   // an overflowed queue holds cap items
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float4 c0 = shadow.at(0, i), c1 = shadow.at(1, i), c2 = shadow.at(2, i), c3 = shadow.at(3, i);
@@ -1559,6 +1583,7 @@ __global__ void k_shadow_split(DevScene s, const float4 *__restrict__ nodes,
 // pixel += L after each sample (integrator.cpp:255-258); with `clear` the
 // next sample starts from L = 0 (the reference keeps L for the whole frame).
 __global__ void k_accumulate(PixelState ps, int64_t n, int clear) {
+    stream_order();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         float4 l = ps.L[i], p = ps.pixel[i];
@@ -1572,6 +1597,7 @@ __global__ void k_accumulate(PixelState ps, int64_t n, int clear) {
 __global__ void k_resolve(PixelState ps, float4 *out, const DevView *__restrict__ views,
                           const FrameConst *__restrict__ fc, int64_t n, float spp, int clamp,
                           float clamp_max) {
+    stream_order();
     const int nv = fc->n_views;
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < n;
          g += (int64_t)gridDim.x * blockDim.x) {
@@ -2752,8 +2778,8 @@ extern "C" int krr_wf_begin_frame_views(krr_wf *wf, int64_t frame_index, const k
 
 static int camera_rays(krr_wf *wf, int64_t p0, int64_t count, cudaStream_t st) {
     ProfScope prof(wf, PS_CAMERA, st);
-    k_camera_rays<<<stage_grid(wf, count), wf->block, 0, st>>>(wf->ps, wf->q(Q_RAY0), wf->d_views,
-                                                               wf->d_frame, p0, count, wf->camera_order);
+    KRR_CUDA(launch_ordered(k_camera_rays, stage_grid(wf, count), wf->block, st, wf->ps, wf->q(Q_RAY0), wf->d_views,
+                                                               wf->d_frame, p0, count, wf->camera_order));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -2768,7 +2794,7 @@ extern "C" int krr_wf_generate_camera_rays(krr_wf *wf, void *stream) {
 
 extern "C" int krr_wf_reset_queues(krr_wf *wf, int32_t depth, void *stream) {
     KRR_TRY(ready(wf));
-    k_reset_queues<<<1, 32, 0, as_stream(stream)>>>(wf->d_counts, depth & 1, depth < 0 ? 1 : 0);
+    KRR_CUDA(launch_ordered(k_reset_queues, 1, 32, as_stream(stream), wf->d_counts, depth & 1, depth < 0 ? 1 : 0));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -2801,8 +2827,8 @@ static TraceLaunch closest_launch(krr_wf *wf, int depth) {
 static int nrc_evaluate_queries(krr_wf *wf, cudaStream_t st) {
     ProfScope prof(wf, PS_CACHE_QUERY, st);
     KRR_TRY(nrc_query_device(wf->nrc, wf->nrc_q_in, wf->nrc_q_count(), wf->n, wf->nrc_q_out, st));
-    k_nrc_apply<<<wf->grid, wf->block, 0, st>>>(wf->nrc_q_out, wf->nrc_q_meta, wf->nrc_q_count(),
-                                                (int)wf->n, wf->ps);
+    KRR_CUDA(launch_ordered(k_nrc_apply, wf->grid, wf->block, st, wf->nrc_q_out, wf->nrc_q_meta, wf->nrc_q_count(),
+                                                (int)wf->n, wf->ps));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -2847,10 +2873,10 @@ static int closest_stage(krr_wf *wf, int depth, cudaStream_t st, bool traced,
     }
     {
         ProfScope prof(wf, PS_ROUTE, st);
-        k_hit_process<<<wf->grid, wf->block, 0, st>>>(wf->scene, rq, wf->hits, wf->q(cur ^ 1),
+        KRR_CUDA(launch_ordered(k_hit_process, wf->grid, wf->block, st, wf->scene, rq, wf->hits, wf->q(cur ^ 1),
                                                       wf->q(Q_MISS), wf->q(Q_HIT_LIGHT), wf->q(Q_SCATTER),
                                                       wf->q(Q_MEDIUM_SAMPLE), wf->medium ? 1 : 0, wf->err(),
-                                                      hook, wf->ps, inline_lights, wf->params.nee);
+                                                      hook, wf->ps, inline_lights, wf->params.nee));
         KRR_CUDA(cudaGetLastError());
     }
     if (wf->nrc && !defer_cache) KRR_TRY(nrc_evaluate_queries(wf, st));
@@ -2876,7 +2902,7 @@ static int trace_shadow_and_next(krr_wf *wf, int depth, cudaStream_t st) {
     l.occluded = wf->occluded;
     set_roots(wf, l, sq, 2, true);   // Shadow: plane 2 = Ld | pixel
     KRR_TRY(launch_trace_mixed(&wf->accel, l, st));
-    k_shadow_resolve<<<wf->grid, wf->block, 0, st>>>(sq, wf->occluded, wf->ps);
+    KRR_CUDA(launch_ordered(k_shadow_resolve, wf->grid, wf->block, st, sq, wf->occluded, wf->ps));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -2884,8 +2910,8 @@ static int trace_shadow_and_next(krr_wf *wf, int depth, cudaStream_t st) {
 extern "C" int krr_wf_handle_hit(krr_wf *wf, void *stream) {
     KRR_TRY(ready(wf));
     ProfScope prof(wf, PS_HIT, as_stream(stream));
-    k_handle_hit<<<wf->grid, wf->block, 0, as_stream(stream)>>>(wf->scene, wf->q(Q_HIT_LIGHT), wf->ps,
-                                                               wf->params.nee);
+    KRR_CUDA(launch_ordered(k_handle_hit, wf->grid, wf->block, as_stream(stream), wf->scene, wf->q(Q_HIT_LIGHT), wf->ps,
+                                                               wf->params.nee));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -2894,8 +2920,8 @@ extern "C" int krr_wf_handle_miss(krr_wf *wf, void *stream) {
     KRR_TRY(ready(wf));
     if (wf->scene.n_infinite == 0) return KRR_OK;
     ProfScope prof(wf, PS_MISS, as_stream(stream));
-    k_handle_miss<<<wf->grid, wf->block, 0, as_stream(stream)>>>(wf->scene, wf->q(Q_MISS), wf->ps,
-                                                                wf->params.nee);
+    KRR_CUDA(launch_ordered(k_handle_miss, wf->grid, wf->block, as_stream(stream), wf->scene, wf->q(Q_MISS), wf->ps,
+                                                                wf->params.nee));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -2916,14 +2942,13 @@ static int scatter_stage(krr_wf *wf, int depth, cudaStream_t st, bool to_tracker
     int cur = depth & 1;
     const Queue tracked = to_tracker ? Queue{wf->media_shadow, (int32_t)wf->qcap, wf->media_shadow_count()}
                                      : Queue{};
-    KRR_CUDA(cudaMemsetAsync(wf->scatter_class_counts(), 0, 4 * sizeof(int32_t), st));
-    k_scatter_classify<<<wf->grid, wf->block, 0, st>>>(wf->scene, wf->q(Q_SCATTER), wf->ps,
+    KRR_CUDA(launch_ordered(k_scatter_classify, wf->grid, wf->block, st, wf->scene, wf->q(Q_SCATTER), wf->ps,
                                                       wf->params.rr, wf->scatter_lists,
-                                                      wf->scatter_class_counts());
-    k_scatter_process<<<wf->grid, wf->block, 0, st>>>(wf->scene, wf->q(Q_SCATTER), wf->scatter_lists,
-                                                     wf->scatter_class_counts(), wf->q(cur ^ 1),
+                                                      wf->scatter_class_counts()));
+    KRR_CUDA(launch_ordered(k_scatter_process, wf->grid, wf->block, st, wf->scene, wf->q(Q_SCATTER), wf->scatter_lists,
+                                                     wf->scatter_class_counts(), wf->scatter_blocks_done(), wf->q(cur ^ 1),
                                                      wf->q(Q_SHADOW), tracked, wf->ps, wf->params.nee,
-                                                     wf->params.rr, resident_grid(wf, 3), wf->err());
+                                                     wf->params.rr, resident_grid(wf, 3), wf->err()));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -2950,7 +2975,7 @@ extern "C" int krr_wf_trace_shadow(krr_wf *wf, void *stream) {
     l.err = wf->accel.d_scratch + 4;
     set_roots(wf, l, sq, 2, false);
     KRR_TRY(launch_trace_any(&wf->accel, l, st));
-    k_shadow_resolve<<<wf->grid, wf->block, 0, st>>>(sq, wf->occluded, wf->ps);
+    KRR_CUDA(launch_ordered(k_shadow_resolve, wf->grid, wf->block, st, sq, wf->occluded, wf->ps));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -3098,10 +3123,7 @@ extern "C" int krr_wf_render(krr_wf *wf, float *d_out, void *stream) {
                     KRR_TRY(krr_wf_handle_miss(wf, stream));
                 }
                 if (depth == loop_depth(wf)) break;
-                if (split) {
-                    KRR_CUDA(cudaMemsetAsync(wf->shadow_tracked_count(), 0, sizeof(int32_t), st));
-                    KRR_CUDA(cudaMemsetAsync(wf->media_shadow_count(), 0, sizeof(int32_t), st));
-                }
+                if (split) KRR_CUDA(cudaMemsetAsync(wf->media_shadow_count(), 0, sizeof(int32_t), st));
                 if (wf->medium) KRR_TRY(launch_medium_scatter(wf, depth, st, split));
                 KRR_TRY(scatter_stage(wf, depth, st, split));
                 if (split) {
@@ -3117,14 +3139,14 @@ extern "C" int krr_wf_render(krr_wf *wf, float *d_out, void *stream) {
         }
         if (wf->nrc && wf->nrc_train) KRR_TRY(nrc_train_frame(wf, st));
         ProfScope prof(wf, PS_RESOLVE, st);
-        k_accumulate<<<wf->grid, wf->block, 0, st>>>(wf->ps, wf->n,
-                                                     wf->params.independent_samples && s + 1 < wf->params.spp);
+        KRR_CUDA(launch_ordered(k_accumulate, wf->grid, wf->block, st, wf->ps, wf->n,
+                                                     wf->params.independent_samples && s + 1 < wf->params.spp));
         KRR_CUDA(cudaGetLastError());
     }
     ProfScope prof(wf, PS_RESOLVE, st);
-    k_resolve<<<wf->grid, wf->block, 0, st>>>(wf->ps, reinterpret_cast<float4 *>(d_out), wf->d_views,
+    KRR_CUDA(launch_ordered(k_resolve, wf->grid, wf->block, st, wf->ps, reinterpret_cast<float4 *>(d_out), wf->d_views,
                                               wf->d_frame, wf->n, (float)wf->params.spp,
-                                              wf->params.enable_clamp, wf->params.clamp_max);
+                                              wf->params.enable_clamp, wf->params.clamp_max));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -3483,11 +3505,11 @@ static int work_order(krr_wf *wf, const Queue &q, int items, cudaStream_t st, co
 int launch_medium_sample(krr_wf *wf, int depth, cudaStream_t st) {
     const int32_t *order = nullptr;
     KRR_TRY(work_order(wf, wf->q(Q_MEDIUM_SAMPLE), 0, st, &order));
-    k_medium_sample<<<resident_grid(wf, 3), wf->block, 0, st>>>(wf->scene, wf->q(Q_MEDIUM_SAMPLE),
+    KRR_CUDA(launch_ordered(k_medium_sample, resident_grid(wf, 3), wf->block, st, wf->scene, wf->q(Q_MEDIUM_SAMPLE),
                                                     wf->q((depth & 1) ^ 1), wf->q(Q_MISS),
                                                     wf->q(Q_HIT_LIGHT), wf->q(Q_SCATTER),
                                                     wf->q(Q_MEDIUM_SCATTER), wf->ps, order,
-                                                    wf->deal_cursor(0), wf->err());
+                                                    wf->deal_cursor(0), wf->err()));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -3522,10 +3544,10 @@ int ensure_split_buffers(krr_wf *wf) {
 
 int launch_medium_scatter(krr_wf *wf, int depth, cudaStream_t st, bool to_tracker) {
     ProfScope prof(wf, PS_MEDIUM_SCATTER, st);
-    k_medium_scatter<<<wf->grid, wf->block, 0, st>>>(wf->scene, wf->q(Q_MEDIUM_SCATTER),
+    KRR_CUDA(launch_ordered(k_medium_scatter, wf->grid, wf->block, st, wf->scene, wf->q(Q_MEDIUM_SCATTER),
                                                      wf->q((depth & 1) ^ 1), wf->q(Q_SHADOW),
                                                      to_tracker ? tracked_queue(wf) : Queue{}, wf->ps,
-                                                     wf->params.nee, wf->err());
+                                                     wf->params.nee, wf->err()));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -3535,8 +3557,7 @@ int launch_medium_scatter(krr_wf *wf, int depth, cudaStream_t st, bool to_tracke
 // own counter and ratio-tracked by k_shadow_tr.
 int launch_trace_shadow_tr(krr_wf *wf, cudaStream_t st) {
     static_assert(kMediumSampleCh >= kShadowCh, "tracked shadow rays need five planes");
-    KRR_CUDA(cudaMemsetAsync(wf->shadow_tracked_count(), 0, sizeof(int32_t), st));
-    KRR_TRY(launch_shadow_split(wf, st, false));
+    KRR_TRY(launch_shadow_split(wf, st, false));   // the tracker leaves its queue empty
     return launch_shadow_tracker(wf, st);
 }
 
@@ -3550,8 +3571,8 @@ int launch_shadow_split(krr_wf *wf, cudaStream_t st, bool media_candidates) {
     int *terr = wf->accel.d_scratch + 4;
     const InstancedView iv = wf->accel.levels == 2 ? instanced_view(&wf->accel) : InstancedView{};
 #define KRR_SHADOW_SPLIT(F, LV)                                                                        \
-    k_shadow_split<F, LV><<<wf->grid, wf->block, 0, st>>>(wf->scene, wf->accel.d_nodes, wf->accel.d_tris, iv, \
-                                                          from, tracked, wf->ps, wf->err(), terr)
+    KRR_CUDA(launch_ordered(k_shadow_split<F, LV>, wf->grid, wf->block, st, wf->scene, wf->accel.d_nodes, wf->accel.d_tris, iv, \
+                                                          from, tracked, wf->ps, wf->err(), terr))
     const bool two = wf->accel.levels == 2, f1 = wf->accel.node_format == 1;
     if (two) { if (f1) KRR_SHADOW_SPLIT(1, 2); else KRR_SHADOW_SPLIT(0, 2); }
     else { if (f1) KRR_SHADOW_SPLIT(1, 1); else KRR_SHADOW_SPLIT(0, 1); }
@@ -3568,8 +3589,8 @@ int launch_shadow_tracker(krr_wf *wf, cudaStream_t st) {
     const int32_t *order = nullptr;
     KRR_TRY(work_order(wf, tracked, 1, st, &order));
 #define KRR_SHADOW_TR(F, LV)                                                                           \
-    k_shadow_tr<F, LV><<<resident_grid(wf, 3), wf->block, 0, st>>>(wf->scene, wf->accel.d_nodes, wf->accel.d_tris, iv, \
-                                                       tracked, wf->ps, order, wf->deal_cursor(1), wf->err(), terr)
+    KRR_CUDA(launch_ordered(k_shadow_tr<F, LV>, resident_grid(wf, 3), wf->block, st, wf->scene, wf->accel.d_nodes, wf->accel.d_tris, iv, \
+                                                       tracked, wf->ps, order, wf->deal_cursor(1), wf->err(), terr))
     const bool two = wf->accel.levels == 2, f1 = wf->accel.node_format == 1;
     if (two) { if (f1) KRR_SHADOW_TR(1, 2); else KRR_SHADOW_TR(0, 2); }
     else { if (f1) KRR_SHADOW_TR(1, 1); else KRR_SHADOW_TR(0, 1); }
