@@ -22,6 +22,7 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -795,6 +796,351 @@ __global__ void k_gather_tris(const float *__restrict__ v, const uint32_t *__res
     leaf_of_prim[p] = (uint32_t)k;
 }
 
+// ------------------------------------------------------------ small trees
+// The instance tree of a two-level structure is rebuilt whenever instances
+// move.  Up to kSmallTree boxes it is built by one block in shared memory:
+// the same Morton codes, radix tree and greedy collapse as above, a warp per
+// wide node (lane c holds child c) instead of a thread with its children in
+// local memory, no allocation and one round trip to the host.  501 instances
+// on GB300: 68 us with the records' kernel, 236 us of kernels and as much in
+// allocations and waits before; new transforms and 518,400 camera rays 1,028
+// and 495 us.
+constexpr int kSmallTree = 1024;
+
+struct SmallTreeShared {
+    unsigned long long key[kSmallTree];
+    uint32_t order[kSmallTree];                       // sorted position -> box
+    float leaf[6][kSmallTree], node[6][kSmallTree];   // lo, hi of sorted leaves and binary nodes
+    uint32_t left[kSmallTree], right[kSmallTree];
+    int par_node[kSmallTree], par_leaf[kSmallTree], flag[kSmallTree];
+    uint32_t item_ref[2][kSmallTree / 2], item_node[2][kSmallTree / 2];
+    float red[32][12];
+    int n_items[2], nodes, tris;
+};
+
+// out: nodes, depth, 1 if a box is not finite (then nothing else is written),
+// unused; then lo, hi of all boxes.
+struct SmallTreeResult {
+    int nodes, depth, bad, pad;
+    float lo[3], hi[3];
+};
+
+__global__ void __launch_bounds__(kSmallTree)
+k_small_tree(const float4 *__restrict__ boxes, int n, int cubic, float4 *nodes, float4 *tris,
+             const TraceInst *__restrict__ inst_new, TraceInst *inst, SmallTreeResult *out) {
+    extern __shared__ __align__(16) unsigned char small_raw[];
+    SmallTreeShared &S = *reinterpret_cast<SmallTreeShared *>(small_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr unsigned kAll = 0xffffffffu;
+
+    // bounds of the centroids and of the boxes, as k_scene_bounds
+    V3 lo = v3(INFINITY), hi = v3(-INFINITY), ce = v3(0.f);
+    float val[12];
+    if (tid < n) {
+        lo = f3(boxes[2 * tid]);
+        hi = f3(boxes[2 * tid + 1]);
+        ce = (lo + hi) * 0.5f;
+    }
+    for (int k = 0; k < 3; ++k) {
+        val[k] = tid < n ? get(ce, k) : INFINITY;
+        val[3 + k] = tid < n ? get(ce, k) : -INFINITY;
+        val[6 + k] = get(lo, k);
+        val[9 + k] = get(hi, k);
+    }
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+        for (int off = 16; off > 0; off >>= 1) {
+            const float y = __shfl_xor_sync(kAll, val[k], off);
+            val[k] = k % 6 < 3 ? fminf(val[k], y) : fmaxf(val[k], y);
+        }
+        if (lane == 0) S.red[warp][k] = val[k];
+    }
+    const bool finite = (isfinite(lo.x) && isfinite(lo.y) && isfinite(lo.z) && isfinite(hi.x) && isfinite(hi.y) &&
+                         isfinite(hi.z)) || tid >= n;
+    const bool bad = __syncthreads_or(!finite) != 0;
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+        val[k] = S.red[lane][k];   // 32 warps
+        for (int off = 16; off > 0; off >>= 1) {
+            const float y = __shfl_xor_sync(kAll, val[k], off);
+            val[k] = k % 6 < 3 ? fminf(val[k], y) : fmaxf(val[k], y);
+        }
+    }
+    if (tid == 0) {
+        out->bad = bad;
+        for (int k = 0; k < 3; ++k) {
+            out->lo[k] = val[6 + k];
+            out->hi[k] = val[9 + k];
+        }
+        S.n_items[0] = 1;
+        S.nodes = 1;
+        S.tris = 0;
+        S.item_node[0][0] = 0u;
+        S.item_ref[0][0] = n > 1 ? 0u : kLeafBit;
+    }
+    if (bad) return;
+    float mag = 0.f, ext = 0.f, emax = 0.f;
+    for (int k = 0; k < 3; ++k) {
+        mag = fmaxf(mag, fmaxf(fabsf(val[6 + k]), fabsf(val[9 + k])));
+        ext = fmaxf(ext, val[9 + k] - val[6 + k]);
+        emax = fmaxf(emax, val[3 + k] - val[k]);
+    }
+    const float margin = ldexpf(mag + ext, -19) + 1e-30f;
+
+    // sort the Morton codes (ties by index, as a stable sort)
+    unsigned long long key = ~0ull;
+    uint32_t idx = (uint32_t)tid;
+    if (tid < n) {
+        uint32_t q[3];
+        for (int k = 0; k < 3; ++k) {
+            const float e = cubic ? emax : val[3 + k] - val[k];
+            const float t = e > 0.f ? (get(ce, k) - val[k]) / e : 0.5f;
+            q[k] = (uint32_t)fminf(fmaxf(t * 2097152.f, 0.f), 2097151.f);
+        }
+        key = (spread21(q[0]) << 2) | (spread21(q[1]) << 1) | spread21(q[2]);
+    }
+    for (int size = 2; size <= kSmallTree; size <<= 1) {
+        for (int step = size >> 1; step > 0; step >>= 1) {
+            unsigned long long okey;
+            uint32_t oidx;
+            if (step >= 32) {
+                S.key[tid] = key;
+                S.order[tid] = idx;
+                __syncthreads();
+                okey = S.key[tid ^ step];
+                oidx = S.order[tid ^ step];
+                __syncthreads();
+            } else {
+                okey = __shfl_xor_sync(kAll, key, step);
+                oidx = __shfl_xor_sync(kAll, idx, step);
+            }
+            const bool up = (tid & size) == 0, first = (tid & step) == 0;
+            const bool less = okey < key || (okey == key && oidx < idx);
+            if (less == (up == first)) {
+                key = okey;
+                idx = oidx;
+            }
+        }
+    }
+    S.key[tid] = key;
+    S.order[tid] = idx;
+    S.flag[tid] = 0;
+    if (tid < n) {
+        const float4 blo = boxes[2 * idx], bhi = boxes[2 * idx + 1];
+        S.leaf[0][tid] = blo.x - margin;
+        S.leaf[1][tid] = blo.y - margin;
+        S.leaf[2][tid] = blo.z - margin;
+        S.leaf[3][tid] = bhi.x + margin;
+        S.leaf[4][tid] = bhi.y + margin;
+        S.leaf[5][tid] = bhi.z + margin;
+    }
+    __syncthreads();
+
+    // radix tree, as k_karras
+    if (tid < n - 1) {
+        const uint64_t *keys = reinterpret_cast<const uint64_t *>(S.key);
+        const int i = tid;
+        const int d = (delta_fn(keys, n, i, i + 1) - delta_fn(keys, n, i, i - 1)) >= 0 ? 1 : -1;
+        const int dmin = delta_fn(keys, n, i, i - d);
+        int lmax = 2;
+        while (delta_fn(keys, n, i, i + lmax * d) > dmin) lmax <<= 1;
+        int l = 0;
+        for (int t = lmax >> 1; t >= 1; t >>= 1)
+            if (delta_fn(keys, n, i, i + (l + t) * d) > dmin) l += t;
+        const int j = i + l * d;
+        const int dnode = delta_fn(keys, n, i, j);
+        int sp = 0, t = l;
+        do {
+            t = (t + 1) >> 1;
+            if (delta_fn(keys, n, i, i + (sp + t) * d) > dnode) sp += t;
+        } while (t > 1);
+        const int gamma = i + sp * d + min(d, 0);
+        const int first = min(i, j), last = max(i, j);
+        if (first == gamma) { S.left[i] = kLeafBit | gamma; S.par_leaf[gamma] = i; }
+        else { S.left[i] = gamma; S.par_node[gamma] = i; }
+        if (last == gamma + 1) { S.right[i] = kLeafBit | (gamma + 1); S.par_leaf[gamma + 1] = i; }
+        else { S.right[i] = gamma + 1; S.par_node[gamma + 1] = i; }
+        if (i == 0) S.par_node[0] = -1;
+    }
+    __syncthreads();
+
+    // boxes bottom-up: the second child to arrive joins the two
+    auto box = [&](uint32_t ref, int k) {
+        return (ref & kLeafBit) ? S.leaf[k][ref & ~kLeafBit] : S.node[k][ref];
+    };
+    if (tid < n && n > 1) {
+        int at = S.par_leaf[tid];
+        while (at >= 0) {
+            __threadfence_block();
+            if (atomicAdd(&S.flag[at], 1) == 0) break;
+            __threadfence_block();
+            const uint32_t l = S.left[at], r = S.right[at];
+            for (int k = 0; k < 3; ++k) {
+                S.node[k][at] = fminf(box(l, k), box(r, k));
+                S.node[3 + k][at] = fmaxf(box(l, 3 + k), box(r, 3 + k));
+            }
+            at = S.par_node[at];
+        }
+    }
+    __syncthreads();
+
+    // wide nodes, level by level, a warp per node
+    int level = 0, depth = 0;
+    while (true) {
+        const int cur = level & 1, m = S.n_items[cur];
+        if (m == 0) break;
+        __syncthreads();   // every warp has read m
+        if (tid == 0) S.n_items[cur ^ 1] = 0;
+        __syncthreads();
+        ++depth;
+        for (int w = warp; w < m; w += kSmallTree / 32) {
+            const uint32_t wnode = S.item_node[cur][w];
+            // open the largest internal child while slots remain
+            uint32_t ref = S.item_ref[cur][w];
+            V3 clo = v3(0.f), chi = v3(0.f);
+            auto load = [&]() {
+                clo = V3{box(ref, 0), box(ref, 1), box(ref, 2)};
+                chi = V3{box(ref, 3), box(ref, 4), box(ref, 5)};
+            };
+            load();
+            int nc = 1;
+            while (nc < 8) {
+                const bool opens = lane < nc && !(ref & kLeafBit);
+                const uint32_t area = opens ? __float_as_uint(half_area(clo, chi)) + 1u : 0u;
+                const uint32_t most = __reduce_max_sync(kAll, area);
+                if (most == 0u) break;
+                const int best = __ffs(__ballot_sync(kAll, area == most)) - 1;
+                const uint32_t r = __shfl_sync(kAll, ref, best);
+                if (lane == best) { ref = S.left[r]; load(); }
+                if (lane == nc) { ref = S.right[r]; load(); }
+                ++nc;
+            }
+            const bool used = lane < nc;
+            const bool internal = used && !(ref & kLeafBit);
+            const unsigned internal_b = __ballot_sync(kAll, internal);
+            V3 nlo = used ? clo : v3(INFINITY), nhi = used ? chi : v3(-INFINITY);
+            for (int off = 4; off > 0; off >>= 1) {
+                nlo = vmin(nlo, V3{__shfl_xor_sync(kAll, nlo.x, off), __shfl_xor_sync(kAll, nlo.y, off),
+                                   __shfl_xor_sync(kAll, nlo.z, off)});
+                nhi = vmax(nhi, V3{__shfl_xor_sync(kAll, nhi.x, off), __shfl_xor_sync(kAll, nhi.y, off),
+                                   __shfl_xor_sync(kAll, nhi.z, off)});
+            }
+            nlo = V3{__shfl_sync(kAll, nlo.x, 0), __shfl_sync(kAll, nlo.y, 0), __shfl_sync(kAll, nlo.z, 0)};
+            nhi = V3{__shfl_sync(kAll, nhi.x, 0), __shfl_sync(kAll, nhi.y, 0), __shfl_sync(kAll, nhi.z, 0)};
+            // octant slots as k_collapse: lane 8 g + c weighs child c for slots 2 g and 2 g + 1
+            uint32_t child_in = 0xffffffffu;   // nibble s: child in slot s, 15 none
+            if (!internal_b && nc <= 4) {
+                for (int c = 0; c < nc; ++c) child_in = (child_in & ~(15u << (4 * c))) | ((uint32_t)c << (4 * c));
+            } else {
+                const V3 pc = (nlo + nhi) * 0.5f, cc = (clo + chi) * 0.5f - pc;
+                const int c = lane & 7;
+                const V3 d = V3{__shfl_sync(kAll, cc.x, c), __shfl_sync(kAll, cc.y, c), __shfl_sync(kAll, cc.z, c)};
+                unsigned done_c = 0u, done_s = 0u;
+                for (int it = 0; it < nc; ++it) {
+                    uint32_t best = 0xffffffffu, at = 0xffffffffu;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int sl = 2 * (lane >> 3) + h;
+                        if (c >= nc || (done_c >> c & 1u) || (done_s >> sl & 1u)) continue;
+                        const float cost = ((sl & 1) ? -d.x : d.x) + ((sl & 2) ? -d.y : d.y) + ((sl & 4) ? -d.z : d.z);
+                        const uint32_t b = __float_as_uint(cost + 0.f);   // -0 as +0
+                        const uint32_t ord = (b & 0x80000000u) ? ~b : b | 0x80000000u;
+                        if (ord < best) { best = ord; at = (uint32_t)(8 * c + sl); }
+                    }
+                    const uint32_t least = __reduce_min_sync(kAll, best);
+                    const uint32_t pick = __reduce_min_sync(kAll, best == least ? at : 0xffffffffu);
+                    const uint32_t pc_ = pick >> 3, ps = pick & 7u;
+                    done_c |= 1u << pc_;
+                    done_s |= 1u << ps;
+                    child_in = (child_in & ~(15u << (4 * ps))) | (pc_ << (4 * ps));
+                }
+            }
+            // lane s takes slot s
+            const int c = lane < 8 ? (int)(child_in >> (4 * lane) & 15u) : 15;
+            const bool have = c < 8;
+            const uint32_t sref = __shfl_sync(kAll, ref, c & 7);
+            const V3 slo = V3{__shfl_sync(kAll, clo.x, c & 7), __shfl_sync(kAll, clo.y, c & 7),
+                              __shfl_sync(kAll, clo.z, c & 7)};
+            const V3 shi = V3{__shfl_sync(kAll, chi.x, c & 7), __shfl_sync(kAll, chi.y, c & 7),
+                              __shfl_sync(kAll, chi.z, c & 7)};
+            const bool s_int = have && !(sref & kLeafBit), s_leaf = have && (sref & kLeafBit);
+            const unsigned imask = __ballot_sync(kAll, s_int), lmask = __ballot_sync(kAll, s_leaf);
+            const unsigned below = (1u << lane) - 1u;
+            int base[3] = {0, 0, 0};   // first child node, first leaf, first item of the next level
+            if (lane == 0) {
+                base[0] = imask ? atomicAdd(&S.nodes, __popc(imask)) : 0;
+                base[1] = lmask ? atomicAdd(&S.tris, __popc(lmask)) : 0;
+                base[2] = imask ? atomicAdd(&S.n_items[cur ^ 1], __popc(imask)) : 0;
+            }
+            for (int k = 0; k < 3; ++k) base[k] = __shfl_sync(kAll, base[k], 0);
+            const int int_rank = __popc(imask & below), tri_off = __popc(lmask & below);
+            uint32_t meta = 0u;
+            if (s_int) {
+                meta = 0x20u | (24u + (uint32_t)lane);
+                S.item_ref[cur ^ 1][base[2] + int_rank] = sref;
+                S.item_node[cur ^ 1][base[2] + int_rank] = (uint32_t)(base[0] + int_rank);
+            } else if (s_leaf) {
+                meta = (1u << 5) | (uint32_t)tri_off;
+                const uint32_t id = S.order[sref & ~kLeafBit];
+                const float4 blo = boxes[2 * id], bhi = boxes[2 * id + 1];
+                float4 *tp = tris + 3 * (size_t)(base[1] + tri_off);
+                tp[0] = make_float4(blo.x, blo.y, blo.z, __uint_as_float(id));
+                tp[1] = make_float4(bhi.x, bhi.y, bhi.z, __uint_as_float(1u));
+                tp[2] = make_float4(bhi.x, bhi.y, bhi.z, 0.f);
+            }
+            // quantised boxes, as write_node_boxes
+            uint32_t word[7];   // lo x, y, z, hi x, y, z, meta of the lane's four slots
+            int ek[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                ek[k] = quant_exponent(get(nhi, k) - get(nlo, k));
+                const float e = ldexpf(1.f, ek[k]), p = get(nlo, k);
+                uint32_t ql = 0xffu, qh = 0u;   // an empty slot: inverted
+                if (have) {
+                    float a = fminf(fmaxf(floorf((get(slo, k) - p) / e), 0.f), 255.f);
+                    float b = fminf(fmaxf(ceilf((get(shi, k) - p) / e), 0.f), 255.f);
+                    while (a > 0.f && fmaf(a, e, p) > get(slo, k)) a -= 1.f;
+                    while (b < 255.f && fmaf(b, e, p) < get(shi, k)) b += 1.f;
+                    ql = (uint32_t)a;
+                    qh = (uint32_t)b;
+                }
+                word[k] = ql << (8 * (lane & 3));
+                word[3 + k] = qh << (8 * (lane & 3));
+            }
+            word[6] = meta << (8 * (lane & 3));
+            uint32_t second[7];
+#pragma unroll
+            for (int k = 0; k < 7; ++k) {
+                word[k] |= __shfl_xor_sync(kAll, word[k], 1);
+                word[k] |= __shfl_xor_sync(kAll, word[k], 2);
+                second[k] = __shfl_sync(kAll, word[k], 4);
+            }
+            if (lane == 0) {
+                const uint32_t ew = (uint32_t)(ek[0] + 127) | ((uint32_t)(ek[1] + 127) << 8) |
+                                    ((uint32_t)(ek[2] + 127) << 16) | ((imask & 0xffu) << 24);
+                auto quad = [&](int a, int b) {
+                    return make_float4(__uint_as_float(word[a]), __uint_as_float(second[a]), __uint_as_float(word[b]),
+                                       __uint_as_float(second[b]));
+                };
+                float4 *np = nodes + 5 * (size_t)wnode;
+                np[0] = make_float4(nlo.x, nlo.y, nlo.z, __uint_as_float(ew));
+                np[1] = make_float4(__uint_as_float((uint32_t)base[0]), __uint_as_float((uint32_t)base[1]),
+                                    __uint_as_float(word[6]), __uint_as_float(second[6]));
+                np[2] = quad(0, 1);
+                np[3] = quad(2, 3);
+                np[4] = quad(4, 5);
+            }
+        }
+        __syncthreads();
+        ++level;
+    }
+    if (tid < n) inst[tid] = inst_new[tid];
+    if (tid == 0) {
+        out->nodes = S.nodes;
+        out->depth = depth;
+    }
+}
+
 __global__ void k_set_mask(float4 *tris, const uint32_t *leaf_of_prim, const uint8_t *mask,
                            int64_t n) {
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1249,6 +1595,11 @@ void accel_free(krr_accel *a) {
     cudaFree(a->d_tris);
     cudaFree(a->d_leaf_of_prim);
     cudaFree(a->d_scratch);
+    cudaFree(a->d_small);
+    a->d_small = nullptr;
+    a->small_cap = 0;
+    cudaFree(a->d_inst_in);
+    a->d_inst_in = nullptr;
     cudaFree(a->stage_rays);
     cudaFree(a->stage_hits);
     cudaFree(a->d_node_bounds);
@@ -1659,6 +2010,50 @@ int accel_build(krr_accel *a, const float *d_v, int64_t n, cudaStream_t s) {
     if (st == KRR_ERR_OVERFLOW && g_treelets > 0 && a->max_depth > kTraversalStack)
         st = build_tree(a, d_v, n, s, 0);
     return st;
+}
+
+int small_tree_limit() { return kSmallTree; }
+
+int accel_build_small(krr_accel *a, const float4 *d_boxes, int n, const TraceInst *d_inst_new, TraceInst *d_inst,
+                      bool *built, cudaStream_t s) {
+    // the settings that k_small_tree builds by
+    *built = n >= 1 && n <= kSmallTree && default_node_format() == 0 && default_max_leaf() == 1 &&
+             default_full_leaf() <= 1 && default_builder() != 1 && g_collapse == 0 && g_treelets == 0;
+    if (!*built) return KRR_OK;
+    const auto t0 = std::chrono::steady_clock::now();
+    static_assert(sizeof(SmallTreeResult) <= 64, "the result shares a small allocation");
+    if (a->small_cap < n || a->n_tris < 1) {
+        accel_free(a);
+        a->small_cap = 0;
+        KRR_CUDA(cudaMalloc(&a->d_scratch, 64));
+        KRR_CUDA(cudaMemsetAsync(a->d_scratch, 0, 64, s));
+        KRR_CUDA(cudaMalloc(&a->d_nodes, kNodeQuads[0] * sizeof(float4) * (size_t)n));
+        KRR_CUDA(cudaMalloc(&a->d_tris, 3 * sizeof(float4) * (size_t)n));
+        KRR_CUDA(cudaMalloc(&a->d_small, 64));
+        a->small_cap = n;
+    }
+    a->node_format = 0;
+    a->max_leaf = a->full_leaf = 1;
+    a->builder = default_builder();
+    a->collapse = a->treelets = 0;
+    static const cudaError_t attr = cudaFuncSetAttribute(k_small_tree, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)sizeof(SmallTreeShared));
+    KRR_CUDA(attr);
+    SmallTreeResult *d_res = reinterpret_cast<SmallTreeResult *>(a->d_small), res{};
+    k_small_tree<<<1, kSmallTree, sizeof(SmallTreeShared), s>>>(d_boxes, n, a->builder != 0, a->d_nodes, a->d_tris,
+                                                                d_inst_new, d_inst, d_res);
+    KRR_CUDA(cudaGetLastError());
+    KRR_CUDA(cudaMemcpyAsync(&res, d_res, sizeof(res), cudaMemcpyDeviceToHost, s));
+    KRR_CUDA(cudaStreamSynchronize(s));
+    if (res.bad) return fail(KRR_ERR_INVALID_ARGUMENT, "triangle vertices are not finite");
+    a->n_tris = n;
+    a->n_nodes = res.nodes;
+    a->max_depth = res.depth;
+    for (int k = 0; k < 3; ++k) { a->scene_lo[k] = res.lo[k]; a->scene_hi[k] = res.hi[k]; }
+    a->build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    if (a->max_depth > kTraversalStack)
+        return fail(KRR_ERR_OVERFLOW, "BVH depth %d exceeds the traversal stack (%d)", a->max_depth, kTraversalStack);
+    return KRR_OK;
 }
 
 // Relocation of one part's tree into the combined arrays: child and

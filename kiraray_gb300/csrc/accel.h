@@ -89,6 +89,14 @@ struct krr_accel {
     std::vector<uint32_t> inst_mask;
     std::vector<int64_t> inst_first;     // global id of each instance's first triangle
     int64_t inst_triangles = 0;
+    // inputs of an instance update on the device, kept between updates: see
+    // build_top_level (instanced.cu); h_inst is read back when it is asked for
+    uint8_t *d_inst_in = nullptr;
+    bool h_inst_stale = false;
+    // a tree of at most small_tree_limit() boxes (accel_build_small): boxes
+    // its buffers hold, and its result's device copy
+    int32_t small_cap = 0;
+    void *d_small = nullptr;
     float4 *d_node_bounds = nullptr;   // 2 per node: lo, hi
     float4 *stage_rays = nullptr;
     float4 *stage_hits = nullptr;
@@ -116,6 +124,13 @@ int accel_build(krr_accel *a, const float *d_vertices, int64_t n_tris, cudaStrea
 // bottom-up over the existing tree; the buffers keep their addresses.
 int accel_refit(krr_accel *a, const float *d_vertices, int64_t n_tris, cudaStream_t stream);
 void accel_free(krr_accel *a);
+// A tree over n boxes (d_boxes: lo, hi) in buffers that a later build of as
+// many keeps; d_inst takes d_inst_new's n records once the tree is built.
+// *built false, and nothing done, for more than small_tree_limit() boxes or
+// build settings that only accel_build knows.
+int accel_build_small(krr_accel *a, const float4 *d_boxes, int n, const TraceInst *d_inst_new, TraceInst *d_inst,
+                      bool *built, cudaStream_t s);
+int small_tree_limit();
 // Several BVHs, one per part of the triangles (part p holds the global ids
 // [part_begin[p], part_begin[p + 1])), in one node and triangle array: part
 // p's tree starts at a->roots[p].  Hits are those of a build per part.  One

@@ -253,13 +253,120 @@ static void invert_3x4(const float *m, float *out) {
     }
 }
 
+// An instance's part of an update that stays: its geometry's box, tree root,
+// id offset and mask (0 for an empty geometry, which also has no box).
+struct InstFixed {
+    float lo[3], hi[3];
+    uint32_t blas_root, id_delta, mask, empty;
+};
+
+// World boxes and records of moved instances, as build_top_level computes
+// them on the host: corners and inverses in double, every operation rounded.
+__global__ void k_instance_records(const InstFixed *__restrict__ fixed, const float *__restrict__ xf, int n,
+                                   float4 *boxes, TraceInst *inst) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const InstFixed F = fixed[i];
+    float mf[12];
+    double m[12];
+    for (int k = 0; k < 12; ++k) {
+        mf[k] = xf[12 * (size_t)i + k];
+        m[k] = (double)mf[k];
+    }
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int c = 0; c < 8 && !F.empty; ++c) {
+        const double p[3] = {(c & 1) ? F.hi[0] : F.lo[0], (c & 2) ? F.hi[1] : F.lo[1], (c & 4) ? F.hi[2] : F.lo[2]};
+        for (int r = 0; r < 3; ++r) {
+            const double w = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(m[4 * r], p[0]), __dmul_rn(m[4 * r + 1], p[1])),
+                                                 __dmul_rn(m[4 * r + 2], p[2])), m[4 * r + 3]);
+            const float f = __double2float_rn(w);
+            // std::min and std::max: a NaN leaves the bound, as on the host
+            if (f < lo[r]) lo[r] = f;
+            if (hi[r] < f) hi[r] = f;
+        }
+    }
+    for (int r = 0; r < 3; ++r) {
+        if (F.empty) lo[r] = hi[r] = 0.f;
+        const float mag = fmaxf(fabsf(lo[r]), fabsf(hi[r]));
+        lo[r] -= ldexpf(mag, -20);
+        hi[r] += ldexpf(mag, -20);
+    }
+    boxes[2 * i] = make_float4(lo[0], lo[1], lo[2], 0.f);
+    boxes[2 * i + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
+    TraceInst I;
+    auto det2 = [](double p, double q, double r, double t) { return __dsub_rn(__dmul_rn(p, q), __dmul_rn(r, t)); };
+    const double a = m[0], b = m[1], c = m[2], d = m[4], e = m[5], f = m[6], g = m[8], h = m[9], k = m[10];
+    const double A = det2(e, k, f, h), B = -det2(d, k, f, g), Cc = det2(d, h, e, g);
+    const double det = __dadd_rn(__dadd_rn(__dmul_rn(a, A), __dmul_rn(b, B)), __dmul_rn(c, Cc));
+    const double id = det != 0.0 ? 1.0 / det : 0.0;
+    const double adj[9] = {A, -det2(b, k, c, h), det2(b, f, c, e), B, det2(a, k, c, g), -det2(a, f, c, d),
+                           Cc, -det2(a, h, b, g), det2(a, e, b, d)};
+    for (int r = 0; r < 3; ++r) {
+        double v[3];
+        for (int j = 0; j < 3; ++j) {
+            v[j] = __dmul_rn(adj[3 * r + j], id);
+            I.inv[4 * r + j] = __double2float_rn(v[j]);
+        }
+        I.inv[4 * r + 3] = __double2float_rn(-__dadd_rn(__dadd_rn(__dmul_rn(v[0], m[3]), __dmul_rn(v[1], m[7])),
+                                                        __dmul_rn(v[2], m[11])));
+    }
+    I.blas_root = F.blas_root;
+    I.id_delta = F.id_delta;
+    I.mask = F.mask;
+    I.pad = 0u;
+    inst[i] = I;
+}
+
+// The device's part of build_top_level for structures whose instance tree
+// fits one block.  a->d_inst_in holds the fixed parts (uploaded once), the
+// transforms, the boxes and the new records.
+static int build_top_level_small(krr_accel *a, bool *built, cudaStream_t s) {
+    const int n = (int)a->inst_geom.size();
+    *built = false;
+    if (n < 1 || n > small_tree_limit()) return KRR_OK;
+    const size_t o_xf = sizeof(InstFixed) * (size_t)n, o_box = (o_xf + 48 * (size_t)n + 15) & ~(size_t)15,
+                 o_rec = o_box + 32 * (size_t)n, bytes = o_rec + sizeof(TraceInst) * (size_t)n;
+    if (!a->d_inst_in) {
+        std::vector<InstFixed> fixed(n);
+        for (int i = 0; i < n; ++i) {
+            const int g = a->inst_geom[i];
+            const bool empty = a->geom_begin[g + 1] == a->geom_begin[g];
+            const float *b = &a->blas->part_bounds[6 * (size_t)g];
+            InstFixed &F = fixed[i];
+            for (int r = 0; r < 3; ++r) { F.lo[r] = b[r]; F.hi[r] = b[3 + r]; }
+            F.blas_root = a->blas->roots.empty() ? 0u : a->blas->roots[g];
+            F.id_delta = (uint32_t)(a->inst_first[i] - a->geom_begin[g]);
+            F.mask = empty ? 0u : a->inst_mask[i];
+            F.empty = empty ? 1u : 0u;
+        }
+        KRR_CUDA(cudaMalloc(&a->d_inst_in, bytes));
+        KRR_CUDA(cudaMemcpyAsync(a->d_inst_in, fixed.data(), o_xf, cudaMemcpyHostToDevice, s));
+        KRR_CUDA(cudaStreamSynchronize(s));
+    }
+    if (!a->d_inst) KRR_CUDA(cudaMalloc(&a->d_inst, n * sizeof(TraceInst)));
+    uint8_t *in = a->d_inst_in;
+    float4 *boxes = reinterpret_cast<float4 *>(in + o_box);
+    TraceInst *rec = reinterpret_cast<TraceInst *>(in + o_rec);
+    KRR_CUDA(cudaMemcpyAsync(in + o_xf, a->inst_xf.data(), 48 * (size_t)n, cudaMemcpyHostToDevice, s));
+    k_instance_records<<<(n + 31) / 32, 32, 0, s>>>(reinterpret_cast<const InstFixed *>(in),
+                                                    reinterpret_cast<const float *>(in + o_xf), n, boxes, rec);
+    KRR_CUDA(cudaGetLastError());
+    a->h_inst.resize(n);
+    a->h_inst_stale = true;
+    return accel_build_small(a->tlas, boxes, n, rec, a->d_inst, built, s);
+}
+
 // The top level over the instances' world boxes (each box given to the
 // builder as the degenerate triangle lo, hi, hi; the builder stores the
 // instance index as the triangle id).  Instance records alongside.
 static int build_top_level(krr_accel *a, cudaStream_t s) {
+    bool built = false;
+    KRR_TRY(build_top_level_small(a, &built, s));
+    if (built) return KRR_OK;
     const int n = (int)a->inst_geom.size();
     std::vector<float> boxes(9 * (size_t)n);
     a->h_inst.assign(n, TraceInst{});
+    a->h_inst_stale = false;
     for (int i = 0; i < n; ++i) {
         const int g = a->inst_geom[i];
         const float *m = &a->inst_xf[12 * (size_t)i];
@@ -433,6 +540,13 @@ extern "C" int krr_accel_instance_inverse(const krr_accel *a, float *h_out, int3
     KRR_CHECK_ARG(a && h_out, "NULL argument");
     KRR_CHECK_ARG(a->levels == 2, "not a two-level structure");
     KRR_CHECK_ARG(n == (int32_t)a->h_inst.size(), "instance count differs");
-    for (int i = 0; i < n; ++i) std::memcpy(h_out + 12 * (size_t)i, a->h_inst[i].inv, 12 * sizeof(float));
+    std::vector<TraceInst> rec;   // the device's, where it computed them
+    if (a->h_inst_stale && n > 0) {
+        rec.resize(n);
+        KRR_CUDA(cudaDeviceSynchronize());
+        KRR_CUDA(cudaMemcpy(rec.data(), a->d_inst, n * sizeof(TraceInst), cudaMemcpyDeviceToHost));
+    }
+    const std::vector<TraceInst> &from = rec.empty() ? a->h_inst : rec;
+    for (int i = 0; i < n; ++i) std::memcpy(h_out + 12 * (size_t)i, from[i].inv, 12 * sizeof(float));
     return KRR_OK;
 }
