@@ -65,21 +65,44 @@ struct Pcg {
         state += initstate;
         next_u32();
     }
-    KRR_HD void advance(int64_t delta) {
-        uint64_t cur_mult = kMult, cur_plus = inc, acc_mult = 1u, acc_plus = 0u;
-        while (delta > 0) {
-            if (delta & 1) {
-                acc_mult *= cur_mult;
-                acc_plus = acc_plus * cur_mult + cur_plus;
-            }
-            cur_plus = (cur_mult + 1) * cur_plus;
-            cur_mult *= cur_mult;
-            delta /= 2;
-        }
-        state = acc_mult * state + acc_plus;
-    }
     KRR_D float get1d() { return __uint_as_float((next_u32() >> 9) | 0x3f800000u) - 1.0f; }
 };
+
+// The generator n steps on: state -> A^n state + (1 + A + ... + A^(n-1)) inc,
+// modulo 2^64.  A pixel starts 256 steps after the one before it: for each
+// hexadecimal digit of the pixel's number the pair (A^n, sum) of 256 x digit x
+// 16^position steps, composed digit by digit, in place of a squaring for each
+// of the 30 bits of n.
+struct PcgJump {
+    uint64_t mult, plus;
+};
+struct PcgPixelJumps {
+    PcgJump digit[8][16];
+};
+constexpr PcgPixelJumps make_pcg_pixel_jumps() {
+    PcgPixelJumps t{};
+    PcgJump one{Pcg::kMult, 1u};
+    for (int k = 0; k < 8; ++k) one = PcgJump{one.mult * one.mult, one.mult * one.plus + one.plus};   // 256 steps
+    for (int p = 0; p < 8; ++p) {
+        PcgJump j{1u, 0u};
+        for (int d = 0; d < 16; ++d) {
+            t.digit[p][d] = j;
+            j = PcgJump{j.mult * one.mult, j.plus * one.mult + one.plus};
+        }
+        one = j;   // 16 of them
+    }
+    return t;
+}
+static __device__ const PcgPixelJumps pcg_pixel_jumps = make_pcg_pixel_jumps();
+
+__device__ __forceinline__ void advance_pixels(Pcg &p, uint32_t pixel) {
+    PcgJump j{1u, 0u};
+    for (int k = 0; pixel; ++k, pixel >>= 4) {
+        const ulonglong2 d = __ldg(reinterpret_cast<const ulonglong2 *>(&pcg_pixel_jumps.digit[k][pixel & 15u]));
+        j = PcgJump{j.mult * d.x, j.plus * d.x + d.y};
+    }
+    p.state = j.mult * p.state + j.plus * p.inc;
+}
 
 // ------------------------------------------------------------ sampling
 // src/render/sampling.h:30-83
