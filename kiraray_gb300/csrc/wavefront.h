@@ -12,6 +12,7 @@ struct DevMesh {
     const float *nrm;       // float3
     const float *uv;        // float2 or nullptr
     const uint32_t *idx;    // uint3
+    const float4 *vert;     // shading's copy, two per vertex: pos, nrm.x | nrm.yz, uv (0 without)
     int32_t material;       // -1 = null material
     int32_t medium_inside, medium_outside;
     int32_t pad;
