@@ -28,7 +28,7 @@ using namespace krr;
 
 namespace krr {
 int accel_set_mask(krr_accel *a, const uint8_t *d_mask, cudaStream_t s);
-int launch_medium_sample(krr_wf *wf, int depth, cudaStream_t s);
+int launch_medium_sample(krr_wf *wf, int depth, cudaStream_t s, bool listed);
 int launch_medium_scatter(krr_wf *wf, int depth, cudaStream_t s, bool to_tracker = false);
 int launch_trace_shadow_tr(krr_wf *wf, cudaStream_t s);
 int launch_shadow_tracker(krr_wf *wf, cudaStream_t s);
@@ -811,6 +811,46 @@ __device__ __forceinline__ V3 miss_radiance(const DevScene &s, const DevScenePar
     return thp * L;
 }
 
+// The roulette and the material lists of generateScatterRays, taken by the
+// kernels that queue its items when nothing happens between them (render()):
+// `lists` null leaves both to k_scatter_classify.  A path that the roulette
+// ends is then neither written to the queue nor read back, and a launch is
+// saved per bounce (512x512 Cornell frame 462 and 444 us, 1080p frame 4.47 and
+// 4.42 ms).
+struct ScatterLists {
+    int32_t *lists, *counts;
+    float rr;
+};
+
+// Whether a path's item goes on to be scattered: as k_scatter_classify, with
+// the pixel's sampler as it stands.
+__device__ __forceinline__ bool scatter_survives(const DevScene &s, const PixelState &ps, uint32_t pixel,
+                                                 uint32_t depth, float rr) {
+    // a path of a scene with a smaller depth than the pass's ends here, as
+    // its scene's pass ends the bounce loop (no draws)
+    if (s.pixel_part && (int)depth >= part_of(s, pixel).max_depth) return false;
+    Pcg rng = load_rng(ps, pixel);
+    if (rng.get1d() < rr) return true;
+    store_rng(ps, pixel, rng);   // the path ends here
+    return false;
+}
+
+// Appends item i to the index list of its material's class, one atomic per
+// class in the warp: classes 0 and 1 fill lists[0..cap) from the front and
+// from the back, classes 2 and 3 fill lists[cap..2 cap) likewise.
+__device__ __forceinline__ void list_item(const DevScene &s, int32_t material, int i, int cap,
+                                          int32_t *__restrict__ lists, int32_t *__restrict__ counts) {
+    const int lane = threadIdx.x & 31;
+    const int cls = min(max(s.materials[material].type, 0), 3);
+    const unsigned peers = __match_any_sync(__activemask(), cls);
+    const int leader = __ffs(peers) - 1;
+    int slot = 0;
+    if (lane == leader) slot = atomicAdd(&counts[cls], __popc(peers));
+    slot = __shfl_sync(peers, slot, leader) + __popc(peers & ((1u << lane) - 1u));
+    int32_t *list = lists + (cls >> 1) * (size_t)cap;
+    list[(cls & 1) ? cap - 1 - slot : slot] = i;
+}
+
 // Routing of a closest hit (__closesthit__/__miss__Closest, device.cu:43-74).
 // Four blocks per SM (64 registers): the mesh gathers are latency-bound.
 // With `inline_lights` (render()) the radiance of a miss and of an emissive
@@ -821,7 +861,7 @@ __device__ __forceinline__ V3 miss_radiance(const DevScene &s, const DevScenePar
 __global__ void __launch_bounds__(kThreads, 4)
 k_hit_process(DevScene s, Queue rq, const float4 *__restrict__ hits, Queue next, Queue miss,
               Queue hitl, Queue scat, Queue msq, int enable_medium, uint32_t *err, NrcHook hook,
-              PixelState ps, int inline_lights, int nee) {
+              PixelState ps, int inline_lights, int nee, ScatterLists sl) {
     stream_order();
     int n = min(*rq.count, rq.cap);   // an overflowed queue holds cap items
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -903,9 +943,10 @@ k_hit_process(DevScene s, Queue rq, const float4 *__restrict__ hits, Queue next,
                 hitl.at(7, j) = c6;
             }
         }
-        if (any(thp)) {
+        if (any(thp) && (!sl.lists || scatter_survives(s, ps, ubits(c5.w), ubits(c4.w), sl.rr))) {
             int j = push_slot(scat.count, scat.cap, err);
             if (j >= 0) {
+                if (sl.lists) list_item(s, sf.material, j, scat.cap, sl.lists, sl.counts);
                 scat.at(0, j) = f4(sf.p, ibits(sf.material));
                 scat.at(1, j) = f4(sf.wo, c4.w);
                 scat.at(2, j) = f4(sf.n, c5.w);
@@ -1032,39 +1073,21 @@ __device__ __forceinline__ void scatter_item(const DevScene &s, const Queue &sca
     }
 }
 
-// generateScatterRays (integrator.cpp:110-164) as two launches over the whole
-// queue.  The first draws every item's Russian roulette (integrator.cpp:
-// 116-118; an ended path stores its sampler and stops) and appends each
-// survivor to the index list of its material class, warp-aggregated: classes
-// 0 and 1 fill `lists[0..n)` from the front and from the back, classes 2 and
-// 3 fill `lists[n..2n)` likewise.  The second walks the four lists in class
-// order with no block barrier, so that a warp runs one BSDF except at the
-// three class boundaries.  Every item is computed exactly as alone (its
-// sampler stream is its pixel's); only the order of the queue pushes changes.
+// generateScatterRays (integrator.cpp:110-164) in two parts.  The first draws
+// every item's Russian roulette (integrator.cpp:116-118; an ended path stores
+// its sampler and stops) and appends each survivor to the index list of its
+// material class: this kernel, or in render() the kernels that queue the
+// items (ScatterLists).  The second walks the four lists in class order with
+// no block barrier, so that a warp runs one BSDF except at the three class
+// boundaries.  Every item is computed exactly as alone (its sampler stream is
+// its pixel's); only the order of the queue pushes changes.
 __global__ void k_scatter_classify(DevScene s, Queue scat, PixelState ps, float rr,
                                    int32_t *__restrict__ lists, int32_t *__restrict__ counts) {
     stream_order();
     const int cap = scat.cap, n = min(*scat.count, cap);
-    const int lane = threadIdx.x & 31;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t pixel = ubits(scat.at(2, i).w);
-        // a path of a scene with a smaller depth than the pass's ends here,
-        // as its scene's pass ends the bounce loop (no draws)
-        if (s.pixel_part && (int)ubits(scat.at(1, i).w) >= part_of(s, pixel).max_depth) continue;
-        Pcg rng = load_rng(ps, pixel);
-        if (rng.get1d() >= rr) {
-            store_rng(ps, pixel, rng);   // the path ends here
-            continue;
-        }
-        const int cls = min(max(s.materials[sbits(scat.at(0, i).w)].type, 0), 3);
-        const unsigned peers = __match_any_sync(__activemask(), cls);
-        const int leader = __ffs(peers) - 1;
-        int slot = 0;
-        if (lane == leader) slot = atomicAdd(&counts[cls], __popc(peers));
-        slot = __shfl_sync(peers, slot, leader) + __popc(peers & ((1u << lane) - 1u));
-        int32_t *list = lists + (cls >> 1) * (size_t)cap;
-        list[(cls & 1) ? cap - 1 - slot : slot] = i;
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        if (scatter_survives(s, ps, ubits(scat.at(2, i).w), ubits(scat.at(1, i).w), rr))
+            list_item(s, sbits(scat.at(0, i).w), i, cap, lists, counts);
 }
 
 // Three blocks per SM (80 registers, 104 bytes spilled): 0.8 % faster per
@@ -1268,7 +1291,8 @@ __device__ __forceinline__ bool delta_track(const DevScene &s, const DevMedium &
 // latency-bound, and the extra warps outweigh a few spilled registers.
 __global__ void __launch_bounds__(kThreads, 3)
 k_medium_sample(DevScene s, Queue msq, Queue next, Queue miss, Queue hitl, Queue scat,
-                Queue mscat, PixelState ps, const int32_t *__restrict__ order, int32_t *cursor, uint32_t *err) {
+                Queue mscat, PixelState ps, const int32_t *__restrict__ order, int32_t *cursor, ScatterLists sl,
+                uint32_t *err) {
     stream_order();
     int n = min(*msq.count, msq.cap);   // an overflowed queue holds cap items
     const Deal deal(cursor);
@@ -1337,8 +1361,10 @@ k_medium_sample(DevScene s, Queue msq, Queue next, Queue miss, Queue hitl, Queue
                 hitl.at(7, j) = f4(pl, c6.w);
             }
         }
+        if (sl.lists && !scatter_survives(s, ps, pixel, depth, sl.rr)) continue;
         int j = push_slot(scat.count, scat.cap, err);
         if (j >= 0) {
+            if (sl.lists) list_item(s, sf.material, j, scat.cap, sl.lists, sl.counts);
             scat.at(0, j) = f4(sf.p, ibits(sf.material));
             scat.at(1, j) = f4(sf.wo, c4.w);
             scat.at(2, j) = f4(sf.n, c5.w);
@@ -2856,6 +2882,19 @@ static int nrc_evaluate_queries(krr_wf *wf, cudaStream_t st) {
     return KRR_OK;
 }
 
+// The scatter items' lists for the kernels that queue them, or none: then
+// scatter_stage makes them.
+static ScatterLists scatter_lists(const krr_wf *wf, bool inline_lists) {
+    return inline_lists ? ScatterLists{wf->scatter_lists, wf->scatter_class_counts(), wf->params.rr} : ScatterLists{};
+}
+
+// Whether render() has the kernels that queue scatter items list them: at a
+// depth that scatters, and unless the media stage between uses the lists'
+// buffer for its work order.
+static bool lists_inline(const krr_wf *wf, int depth) {
+    return depth < loop_depth(wf) && !(wf->medium && wf->media_order);
+}
+
 // Routing of the closest hits of ray queue `depth` (already traced into
 // wf->hits when `traced`).  With a cache attached, the paths that stop at it
 // are evaluated and their radiance added here, or, with `in_render`, left in
@@ -2863,7 +2902,7 @@ static int nrc_evaluate_queries(krr_wf *wf, cudaStream_t st) {
 // without media also adds miss and emission radiance in the routing kernel
 // (render() then skips handleHit/handleMiss).
 static int closest_stage(krr_wf *wf, int depth, cudaStream_t st, bool traced,
-                         bool in_render = false) {
+                         bool in_render) {
     // In render() the radiance of misses and emissive hits of rays outside
     // every medium is added here; rays inside a medium go to the medium
     // stage, which queues theirs for handleHit/handleMiss.  A path has one
@@ -2899,7 +2938,8 @@ static int closest_stage(krr_wf *wf, int depth, cudaStream_t st, bool traced,
         KRR_CUDA(launch_ordered(k_hit_process, wf->grid, wf->block, st, wf->scene, rq, wf->hits, wf->q(cur ^ 1),
                                                       wf->q(Q_MISS), wf->q(Q_HIT_LIGHT), wf->q(Q_SCATTER),
                                                       wf->q(Q_MEDIUM_SAMPLE), wf->medium ? 1 : 0, wf->err(),
-                                                      hook, wf->ps, inline_lights, wf->params.nee));
+                                                      hook, wf->ps, inline_lights, wf->params.nee,
+                                                      scatter_lists(wf, in_render && lists_inline(wf, depth))));
         KRR_CUDA(cudaGetLastError());
     }
     if (wf->nrc && !defer_cache) KRR_TRY(nrc_evaluate_queries(wf, st));
@@ -2908,7 +2948,7 @@ static int closest_stage(krr_wf *wf, int depth, cudaStream_t st, bool traced,
 
 extern "C" int krr_wf_trace_closest(krr_wf *wf, int32_t depth, void *stream) {
     KRR_TRY(ready(wf));
-    return closest_stage(wf, depth, as_stream(stream), false);
+    return closest_stage(wf, depth, as_stream(stream), false, false);
 }
 
 // Shadow rays of bounce `depth` and the closest-hit rays of bounce depth+1
@@ -2960,14 +3000,15 @@ static int resident_grid(const krr_wf *wf, int per_sm) {
 
 // generateScatterRays; with `to_tracker` the shadow rays of scenes with
 // media go to their own queue for k_shadow_split (split_shadows()).
-static int scatter_stage(krr_wf *wf, int depth, cudaStream_t st, bool to_tracker) {
+// `listed`: the items' lists are there (scatter_lists).
+static int scatter_stage(krr_wf *wf, int depth, cudaStream_t st, bool to_tracker, bool listed) {
     ProfScope prof(wf, PS_SCATTER, st);
     int cur = depth & 1;
     const Queue tracked = to_tracker ? Queue{wf->media_shadow, (int32_t)wf->qcap, wf->media_shadow_count()}
                                      : Queue{};
-    KRR_CUDA(launch_ordered(k_scatter_classify, wf->grid, wf->block, st, wf->scene, wf->q(Q_SCATTER), wf->ps,
-                                                      wf->params.rr, wf->scatter_lists,
-                                                      wf->scatter_class_counts()));
+    if (!listed)
+        KRR_CUDA(launch_ordered(k_scatter_classify, wf->grid, wf->block, st, wf->scene, wf->q(Q_SCATTER), wf->ps,
+                                wf->params.rr, wf->scatter_lists, wf->scatter_class_counts()));
     KRR_CUDA(launch_ordered(k_scatter_process, wf->grid, wf->block, st, wf->scene, wf->q(Q_SCATTER), wf->scatter_lists,
                                                      wf->scatter_class_counts(), wf->scatter_blocks_done(), wf->q(cur ^ 1),
                                                      wf->q(Q_SHADOW), tracked, wf->ps, wf->params.nee,
@@ -2978,7 +3019,7 @@ static int scatter_stage(krr_wf *wf, int depth, cudaStream_t st, bool to_tracker
 
 extern "C" int krr_wf_generate_scatter_rays(krr_wf *wf, int32_t depth, void *stream) {
     KRR_TRY(ready(wf));
-    return scatter_stage(wf, depth, as_stream(stream), false);
+    return scatter_stage(wf, depth, as_stream(stream), false, false);
 }
 
 extern "C" int krr_wf_trace_shadow(krr_wf *wf, void *stream) {
@@ -3007,7 +3048,7 @@ extern "C" int krr_wf_sample_medium_interaction(krr_wf *wf, int32_t depth, void 
     KRR_TRY(ready(wf));
     if (!wf->medium) return KRR_OK;
     ProfScope prof(wf, PS_MEDIUM_SAMPLE, as_stream(stream));
-    return launch_medium_sample(wf, depth, as_stream(stream));
+    return launch_medium_sample(wf, depth, as_stream(stream), false);
 }
 
 extern "C" int krr_wf_sample_medium_scattering(krr_wf *wf, int32_t depth, void *stream) {
@@ -3141,14 +3182,17 @@ extern "C" int krr_wf_render(krr_wf *wf, float *d_out, void *stream) {
                 KRR_TRY(krr_wf_reset_queues(wf, depth, stream));
                 KRR_TRY(closest_stage(wf, depth, st, traced, true));
                 if (wf->medium) {
-                    KRR_TRY(krr_wf_sample_medium_interaction(wf, depth, stream));
+                    {
+                        ProfScope prof(wf, PS_MEDIUM_SAMPLE, st);
+                        KRR_TRY(launch_medium_sample(wf, depth, st, lists_inline(wf, depth)));
+                    }
                     KRR_TRY(krr_wf_handle_hit(wf, stream));
                     KRR_TRY(krr_wf_handle_miss(wf, stream));
                 }
                 if (depth == loop_depth(wf)) break;
                 if (split) KRR_CUDA(cudaMemsetAsync(wf->media_shadow_count(), 0, sizeof(int32_t), st));
                 if (wf->medium) KRR_TRY(launch_medium_scatter(wf, depth, st, split));
-                KRR_TRY(scatter_stage(wf, depth, st, split));
+                KRR_TRY(scatter_stage(wf, depth, st, split, lists_inline(wf, depth)));
                 if (split) {
                     ProfScope prof(wf, PS_SHADOW, st);
                     KRR_TRY(launch_shadow_split(wf, st, true));
@@ -3527,14 +3571,14 @@ static int work_order(krr_wf *wf, const Queue &q, int items, cudaStream_t st, co
     return KRR_OK;
 }
 
-int launch_medium_sample(krr_wf *wf, int depth, cudaStream_t st) {
+int launch_medium_sample(krr_wf *wf, int depth, cudaStream_t st, bool listed) {
     const int32_t *order = nullptr;
     KRR_TRY(work_order(wf, wf->q(Q_MEDIUM_SAMPLE), 0, st, &order));
     KRR_CUDA(launch_ordered(k_medium_sample, resident_grid(wf, 3), wf->block, st, wf->scene, wf->q(Q_MEDIUM_SAMPLE),
                                                     wf->q((depth & 1) ^ 1), wf->q(Q_MISS),
                                                     wf->q(Q_HIT_LIGHT), wf->q(Q_SCATTER),
                                                     wf->q(Q_MEDIUM_SCATTER), wf->ps, order,
-                                                    wf->deal_cursor(0), wf->err()));
+                                                    wf->deal_cursor(0), scatter_lists(wf, listed), wf->err()));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
