@@ -96,6 +96,7 @@ struct krr_wf {
     int32_t levels = 1;                    // 1: flattened instances, 2: two-level structure
     int32_t mk_reorder = 1;                // megakernel: reorder paths by hit class per bounce
     int32_t media_order = 0;               // 1: tracking kernels take their items by work class
+    bool grey_media = false;               // every medium has three equal channels
     int32_t camera_order = 1;              // 1: camera rays in 8x8 pixel tiles, 0: row-major
     // stage timers (krr_wf_set_profiling): event pairs recorded since the
     // last krr_wf_profile_read, and a pool of spare events
@@ -1289,6 +1290,11 @@ __device__ __forceinline__ bool delta_track(const DevScene &s, const DevMedium &
 // sampleMediumInteraction, medium.cpp:13-103 (the medium has no emission).
 // Three blocks of 256 per SM (at most 80 registers): the tracking loops are
 // latency-bound, and the extra warps outweigh a few spilled registers.
+// GREY: all of the pass's media are grey (krr_wf_set_scenes), so that every
+// walk is (the path probabilities start grey and only media could colour
+// them): less to fetch and to keep in registers, here and in k_shadow_tr
+// (1024x1024 volume frame 5.57 and 5.46 ms).
+template <bool GREY>
 __global__ void __launch_bounds__(kThreads, 3)
 k_medium_sample(DevScene s, Queue msq, Queue next, Queue miss, Queue hitl, Queue scat,
                 Queue mscat, PixelState ps, const int32_t *__restrict__ order, int32_t *cursor, ScatterLists sl,
@@ -1313,7 +1319,7 @@ k_medium_sample(DevScene s, Queue msq, Queue next, Queue miss, Queue hitl, Queue
         int ch = main_index(ps.L[pixel].w);
         const DevMedium &m = s.media[medium];
         bool scattered;
-        if (grey(m) && grey(pu) && grey(pl)) {
+        if (GREY || (grey(m) && grey(pu) && grey(pl))) {
             float u1 = pu.x, l1 = pl.x;
             scattered = delta_track(s, m, o, dir, tmax_hit, rng, ch, thp, u1, l1, medium, depth, pixel, time, mscat, err);
             pu = v3(u1);
@@ -1493,7 +1499,7 @@ __device__ __forceinline__ float4 shadow_trace(const InstancedView &iv, const fl
     else return traverse_ray<ANY, FMT, MASKED>(nodes, tris, o, d, 0.f, tmax, trace_err, root);
 }
 
-template <int FMT, int LEVELS>
+template <int FMT, int LEVELS, bool GREY>
 __global__ void __launch_bounds__(kThreads, 3)
 k_shadow_tr(DevScene s, const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
             InstancedView iv, Queue shadow, PixelState ps, const int32_t *__restrict__ order,
@@ -1532,7 +1538,7 @@ k_shadow_tr(DevScene s, const float4 *__restrict__ nodes, const float4 *__restri
             if (medium >= 0) {
                 float t_end = visible ? tmax : length(sf.p - o) / length(d);
                 const DevMedium &m = s.media[medium];
-                if (grey(m) && grey(T_ray) && grey(pu) && grey(pl)) {
+                if (GREY || (grey(m) && grey(T_ray) && grey(pu) && grey(pl))) {
                     float T1 = T_ray.x, u1 = pu.x, l1 = pl.x;
                     ratio_track(s, m, o, d, t_end, rng, ch, T1, u1, l1, err);
                     T_ray = v3(T1);
@@ -2527,6 +2533,7 @@ extern "C" int krr_wf_set_scenes(krr_wf *wf, const krr_scene_desc *scenes, int32
 
     // media
     std::vector<DevMedium> media(med0[n_scenes]);
+    wf->grey_media = true;
     for (int p = 0; p < n_scenes; ++p)
         for (int i = 0; i < scenes[p].n_media; ++i) {
             const krr_medium_desc &m = scenes[p].media[i];
@@ -2566,6 +2573,9 @@ extern "C" int krr_wf_set_scenes(krr_wf *wf, const krr_scene_desc *scenes, int32
                 KRR_CUDA(cudaGetLastError());
                 d.majorant = maj;
             }
+            // bit for bit, as the kernels' test
+            wf->grey_media = wf->grey_media && std::memcmp(&d.sigma_t[0], &d.sigma_t[1], 2 * sizeof(float)) == 0 &&
+                             std::memcmp(&d.albedo[0], &d.albedo[1], 2 * sizeof(float)) == 0;
             media[med0[p] + i] = d;
         }
     KRR_TRY(dev_upload(wf, const_cast<DevMedium **>(&s.media), media.data(), media.size()));
@@ -3574,7 +3584,7 @@ static int work_order(krr_wf *wf, const Queue &q, int items, cudaStream_t st, co
 int launch_medium_sample(krr_wf *wf, int depth, cudaStream_t st, bool listed) {
     const int32_t *order = nullptr;
     KRR_TRY(work_order(wf, wf->q(Q_MEDIUM_SAMPLE), 0, st, &order));
-    KRR_CUDA(launch_ordered(k_medium_sample, resident_grid(wf, 3), wf->block, st, wf->scene, wf->q(Q_MEDIUM_SAMPLE),
+    KRR_CUDA(launch_ordered(wf->grey_media ? k_medium_sample<true> : k_medium_sample<false>, resident_grid(wf, 3), wf->block, st, wf->scene, wf->q(Q_MEDIUM_SAMPLE),
                                                     wf->q((depth & 1) ^ 1), wf->q(Q_MISS),
                                                     wf->q(Q_HIT_LIGHT), wf->q(Q_SCATTER),
                                                     wf->q(Q_MEDIUM_SCATTER), wf->ps, order,
@@ -3658,7 +3668,7 @@ int launch_shadow_tracker(krr_wf *wf, cudaStream_t st) {
     const int32_t *order = nullptr;
     KRR_TRY(work_order(wf, tracked, 1, st, &order));
 #define KRR_SHADOW_TR(F, LV)                                                                           \
-    KRR_CUDA(launch_ordered(k_shadow_tr<F, LV>, resident_grid(wf, 3), wf->block, st, wf->scene, wf->accel.d_nodes, wf->accel.d_tris, iv, \
+    KRR_CUDA(launch_ordered(wf->grey_media ? k_shadow_tr<F, LV, true> : k_shadow_tr<F, LV, false>, resident_grid(wf, 3), wf->block, st, wf->scene, wf->accel.d_nodes, wf->accel.d_tris, iv, \
                                                        tracked, wf->ps, order, wf->deal_cursor(1), wf->err(), terr))
     const bool two = wf->accel.levels == 2, f1 = wf->accel.node_format == 1;
     if (two) { if (f1) KRR_SHADOW_TR(1, 2); else KRR_SHADOW_TR(0, 2); }
