@@ -1175,10 +1175,11 @@ __device__ __forceinline__ void store_result(const TraceLaunch &L, bool any_ray,
     if (MODE == 1 || (MODE == 2 && any_ray)) {
         L.occluded[ray_id] = prim == kCutRay ? 0xFF : (prim != KRR_MISS ? 1 : 0);
     } else {
-        L.hits[ray_id] = prim < kCutRay
-                             ? make_float4(t, b1, b2, __uint_as_float(prim))
-                             : make_float4(prim == kCutRay ? __int_as_float(0x7fffffff) : INFINITY, 0.f, 0.f,
-                                           __uint_as_float(KRR_MISS));
+        float4 *hits = MODE == 3 && any_ray ? L.hits2 : L.hits;
+        hits[ray_id] = prim < kCutRay
+                           ? make_float4(t, b1, b2, __uint_as_float(prim))
+                           : make_float4(prim == kCutRay ? __int_as_float(0x7fffffff) : INFINITY, 0.f, 0.f,
+                                         __uint_as_float(KRR_MISS));
     }
 }
 
@@ -1322,7 +1323,8 @@ __device__ __forceinline__ void team_phase(const float4 *__restrict__ nodes, con
     }
 }
 
-// MODE 0: closest hit, 1: any hit, 2: mixed (any-hit set, then closest set).
+// MODE 0: closest hit, 1: any hit, 2: mixed (any-hit set, then closest set),
+// 3: pair (two closest-hit sets; any_ray marks the first one's rays).
 template <int MODE, bool STATS, int FMT>
 __device__ __forceinline__ void trace_body(const float4 *__restrict__ nodes,
                                            const float4 *__restrict__ tris, const TraceLaunch &L,
@@ -1331,7 +1333,7 @@ __device__ __forceinline__ void trace_body(const float4 *__restrict__ nodes,
     const int lane = threadIdx.x & 31;
     // queue counts are clamped to the queue capacity (a queue that overflowed
     // has its flag raised and a count above its storage)
-    const int64_t n_any = MODE == 2 ? min((int64_t)*L.d_any_count, L.n) : 0;
+    const int64_t n_any = MODE >= 2 ? min((int64_t)*L.d_any_count, L.n) : 0;
     const int64_t n = (L.d_count ? min((int64_t)*L.d_count, L.n) : L.n) + n_any;
     bool any_ray = MODE == 1;
     uint2 stack[kTraversalStack];
@@ -1375,7 +1377,7 @@ __device__ __forceinline__ void trace_body(const float4 *__restrict__ nodes,
                 int64_t idx = base + rank;
                 if (idx < n) {
                     const float4 *po = L.ray_o, *pd = L.ray_d;
-                    if (MODE == 2) {
+                    if (MODE >= 2) {
                         any_ray = idx < n_any;
                         if (any_ray) { po = L.any_o; pd = L.any_d; }
                         else idx -= n_any;
@@ -1383,7 +1385,7 @@ __device__ __forceinline__ void trace_body(const float4 *__restrict__ nodes,
                     ray_id = idx;
                     uint32_t root = 0;
                     if (L.roots) {
-                        const float4 *pp = (MODE == 2 && any_ray) ? L.any_pix : L.ray_pix;
+                        const float4 *pp = (MODE >= 2 && any_ray) ? L.any_pix : L.ray_pix;
                         root = L.roots[L.pixel_part[__float_as_uint(pp[idx * L.ray_stride].w)]];
                     }
                     float4 ro = po[idx * L.ray_stride];
@@ -1442,7 +1444,7 @@ __device__ __forceinline__ void trace_body(const float4 *__restrict__ nodes,
             float b1, b2;
             float t = tri_test(r, v0, v1, v2, b1, b2);
             uint32_t gid = __float_as_uint(v0.w);
-            if (any_ray) {
+            if (MODE != 3 && any_ray) {
                 if (t > r.tmin && t <= tmax && __float_as_uint(v1.w) != 0u) {
                     best_prim = gid;
                     done = true;
@@ -1491,26 +1493,27 @@ k_trace(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, Trace
     trace_body<MODE, STATS, FMT>(nodes, tris, L, stats);
 }
 
-// The mixed launch is held to the closest-hit kernel's 8 blocks per SM (the
-// grid is sized for that occupancy).
-template <int FMT>
+// The mixed and pair launches are held to the closest-hit kernel's 8 blocks
+// per SM (the grid is sized for that occupancy).
+template <int MODE, int FMT>
 __global__ void __launch_bounds__(kTraceThreads, FMT != 1 ? 8 : 1)
 k_trace_mixed(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, TraceLaunch L) {
     stream_order();
-    trace_body<2, false, FMT>(nodes, tris, L, nullptr);
+    trace_body<MODE, false, FMT>(nodes, tris, L, nullptr);
 }
 
 int g_grid_size = 0;
 
 // An empty scene: every ray misses (MODE as k_trace).
 __global__ void k_all_miss(TraceLaunch L, int mode) {
-    const int64_t n_any = mode == 2 ? min((int64_t)*L.d_any_count, L.n) : 0;
+    const int64_t n_any = mode >= 2 ? min((int64_t)*L.d_any_count, L.n) : 0;
     const int64_t n = (L.d_count ? min((int64_t)*L.d_count, L.n) : L.n) + n_any;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
-        const bool any = mode == 1 || (mode == 2 && i < n_any);
-        if (any) L.occluded[i] = 0;
-        else L.hits[mode == 2 ? i - n_any : i] = make_float4(INFINITY, 0.f, 0.f, __uint_as_float(KRR_MISS));
+        const float4 miss = make_float4(INFINITY, 0.f, 0.f, __uint_as_float(KRR_MISS));
+        if (mode == 3 && i < n_any) L.hits2[i] = miss;
+        else if (mode == 1 || i < n_any) L.occluded[i] = 0;
+        else L.hits[i - n_any] = miss;
     }
 }
 
@@ -1545,24 +1548,25 @@ static int launch_trace(const krr_accel *a, const TraceLaunch &l, cudaStream_t s
     int grid = traversal_grid_size();
     // a set that is dealt out evenly (trace_body) needs no work counter; a
     // small one of known size no more warps than rays
-    const int64_t most = MODE == 2 ? 2 * l.n : l.n;
+    const int64_t most = MODE >= 2 ? 2 * l.n : l.n;
     const bool dealt = !STATS && lt.teams && a->levels != 2 && a->node_format != 1 &&
                        most <= (int64_t)grid * kTraceThreads;
-    if (dealt && MODE != 2 && !l.d_count)
+    if (dealt && MODE < 2 && !l.d_count)
         grid = (int)std::min<int64_t>(grid, (l.n + kTraceThreads / 32 - 1) / (kTraceThreads / 32));
     if (!dealt) KRR_CUDA(cudaMemsetAsync(l.counter, 0, sizeof(unsigned long long), s));
     if (a->levels == 2) {
         KRR_CHECK_ARG(!STATS, "the counter replay takes a one-level structure");
+        KRR_CHECK_ARG(MODE != 3, "the pair launch takes a one-level structure");
         return launch_trace_instanced(a, lt, MODE, s);
     }
     const bool single = a->max_leaf == 1 && a->full_leaf == 1;
-    if constexpr (MODE == 2) {
+    if constexpr (MODE >= 2) {
         if (a->node_format == 1)
-            KRR_CUDA(launch_ordered(k_trace_mixed<1>, grid, kTraceThreads, s, a->d_nodes, a->d_tris, lt));
+            KRR_CUDA(launch_ordered(k_trace_mixed<MODE, 1>, grid, kTraceThreads, s, a->d_nodes, a->d_tris, lt));
         else if (single)
-            KRR_CUDA(launch_ordered(k_trace_mixed<2>, grid, kTraceThreads, s, a->d_nodes, a->d_tris, lt));
+            KRR_CUDA(launch_ordered(k_trace_mixed<MODE, 2>, grid, kTraceThreads, s, a->d_nodes, a->d_tris, lt));
         else
-            KRR_CUDA(launch_ordered(k_trace_mixed<0>, grid, kTraceThreads, s, a->d_nodes, a->d_tris, lt));
+            KRR_CUDA(launch_ordered(k_trace_mixed<MODE, 0>, grid, kTraceThreads, s, a->d_nodes, a->d_tris, lt));
     } else {
         if (a->node_format == 1)
             KRR_CUDA(launch_ordered(k_trace<MODE, STATS, 1>, grid, kTraceThreads, s, a->d_nodes, a->d_tris, lt, stats));
@@ -1583,6 +1587,9 @@ int launch_trace_any(const krr_accel *a, const TraceLaunch &l, cudaStream_t s) {
 }
 int launch_trace_mixed(const krr_accel *a, const TraceLaunch &l, cudaStream_t s) {
     return launch_trace<2, false>(a, l, s);
+}
+int launch_trace_pair(const krr_accel *a, const TraceLaunch &l, cudaStream_t s) {
+    return launch_trace<3, false>(a, l, s);
 }
 int launch_trace_stats(const krr_accel *a, const TraceLaunch &l, bool any,
                        unsigned long long *d_stats, cudaStream_t s) {

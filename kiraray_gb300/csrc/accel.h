@@ -156,9 +156,12 @@ struct TraceLaunch {
     // Mixed launches only: an any-hit ray set traced in the same launch as
     // the closest-hit set above (same stride); its rays take indices
     // [0, *d_any_count) of the shared work counter.
+    // Pair launches: the second set is one of closest-hit rays too, its hits
+    // go to hits2.
     const float4 *any_o;
     const float4 *any_d;
     const int *d_any_count;
+    float4 *hits2;
     // Several BVHs (accel_build_parts): ray i starts at roots[pixel_part[p]]
     // with p the pixel id in ray_pix[i * ray_stride].w (any_pix for the
     // any-hit set); roots == nullptr: every ray starts at node 0.
@@ -170,6 +173,7 @@ struct TraceLaunch {
 
 int launch_trace_closest(const krr_accel *a, const TraceLaunch &l, cudaStream_t s);
 int launch_trace_any(const krr_accel *a, const TraceLaunch &l, cudaStream_t s);
+int launch_trace_pair(const krr_accel *a, const TraceLaunch &l, cudaStream_t s);   // one level
 // One launch for an any-hit set (any_o/any_d -> occluded) and a closest-hit
 // set (ray_o/ray_d -> hits): the two sets share one persistent grid, so the
 // latency tail of the longest ray is paid once.
