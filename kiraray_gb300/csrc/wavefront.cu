@@ -594,10 +594,14 @@ __device__ __forceinline__ int64_t tile_pixel(int64_t i, int w, int h) {
 // Each view's positions map onto its own pixels, so waves (ranges of
 // positions) still cover every pixel once; a path depends only on its
 // pixel, so frames are the same in either order.
+// `counts`: the queue sizes, all set to 0 but this one's (null: left alone).
 __global__ void k_camera_rays(PixelState ps, Queue rq, const DevView *__restrict__ views,
-                              const FrameConst *__restrict__ fc, int64_t p0, int64_t n, int tiled) {
+                              const FrameConst *__restrict__ fc, int64_t p0, int64_t n, int tiled, int32_t *counts) {
     stream_order();
-    if (blockIdx.x == 0 && threadIdx.x == 0) *rq.count = (int32_t)n;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        for (int k = 0; counts && k < Q_COUNT; ++k) counts[k] = 0;
+        *rq.count = (int32_t)n;
+    }
     const int nv = fc->n_views;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
          q += (int64_t)gridDim.x * blockDim.x) {
@@ -821,6 +825,7 @@ __device__ __forceinline__ V3 miss_radiance(const DevScene &s, const DevScenePar
 struct ScatterLists {
     int32_t *lists, *counts;
     float rr;
+    int32_t *shadow_count;   // set to 0 by k_hit_process (null: left alone)
 };
 
 // Whether a path's item goes on to be scattered: as k_scatter_classify, with
@@ -864,6 +869,7 @@ k_hit_process(DevScene s, Queue rq, const float4 *__restrict__ hits, Queue next,
               Queue hitl, Queue scat, Queue msq, int enable_medium, uint32_t *err, NrcHook hook,
               PixelState ps, int inline_lights, int nee, ScatterLists sl) {
     stream_order();
+    if (sl.shadow_count && blockIdx.x == 0 && threadIdx.x == 0) *sl.shadow_count = 0;
     int n = min(*rq.count, rq.cap);   // an overflowed queue holds cap items
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float4 h = hits[i];
@@ -1104,7 +1110,7 @@ __global__ void k_scatter_classify(DevScene s, Queue scat, PixelState ps, float 
 // frames at 241x135 1,012 and 934 us, at 1920x1080 4.91 and 4.76 ms.
 __global__ void __launch_bounds__(kThreads, 3)
 k_scatter_process(DevScene s, Queue scat, const int32_t *__restrict__ lists,
-                  int32_t *counts, int32_t *blocks_done, Queue next, Queue shadow, Queue tracked,
+                  int32_t *counts, int32_t *blocks_done, int32_t *rays_done, Queue next, Queue shadow, Queue tracked,
                   PixelState ps, int nee, float rr, int resident, uint32_t *err) {
     stream_order();
     const int cap = scat.cap;
@@ -1140,12 +1146,17 @@ k_scatter_process(DevScene s, Queue scat, const int32_t *__restrict__ lists,
             scatter_item(s, scat, i, rng, next, shadow, tracked, ps, nee, rr, light, bounce, err);
         }
     }
-    // the last block leaves the class counts 0 for the next launch of
-    // k_scatter_classify
+    // the last block leaves the class counts 0 for the next items' lists and,
+    // in render() without media (`rays_done`), empties this queue and the one
+    // of the rays that led here
     __syncthreads();
     if (threadIdx.x == 0 && atomicAdd(blocks_done, 1) == (int)gridDim.x - 1) {
         for (int k = 0; k < 4; ++k) counts[k] = 0;
         *blocks_done = 0;
+        if (rays_done) {
+            *rays_done = 0;
+            *scat.count = 0;
+        }
     }
 }
 
@@ -2842,10 +2853,11 @@ extern "C" int krr_wf_begin_frame_views(krr_wf *wf, int64_t frame_index, const k
     return begin_frame_common(wf, frame_index, nullptr, views, n_views, as_stream(stream));
 }
 
-static int camera_rays(krr_wf *wf, int64_t p0, int64_t count, cudaStream_t st) {
+static int camera_rays(krr_wf *wf, int64_t p0, int64_t count, cudaStream_t st, bool reset) {
     ProfScope prof(wf, PS_CAMERA, st);
     KRR_CUDA(launch_ordered(k_camera_rays, stage_grid(wf, count), wf->block, st, wf->ps, wf->q(Q_RAY0), wf->d_views,
-                                                               wf->d_frame, p0, count, wf->camera_order));
+                                                               wf->d_frame, p0, count, wf->camera_order,
+                                                               reset ? wf->d_counts : nullptr));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
@@ -2855,7 +2867,7 @@ extern "C" int krr_wf_generate_camera_rays(krr_wf *wf, void *stream) {
     KRR_CHECK_ARG(wf->qcap == wf->n,
                   "the stage entry points trace every pixel at once: the queue capacity must be the "
                   "pixel count (krr_wf_set_launch with wave 0)");
-    return camera_rays(wf, 0, wf->n, as_stream(stream));
+    return camera_rays(wf, 0, wf->n, as_stream(stream), false);
 }
 
 extern "C" int krr_wf_reset_queues(krr_wf *wf, int32_t depth, void *stream) {
@@ -2902,7 +2914,9 @@ static int nrc_evaluate_queries(krr_wf *wf, cudaStream_t st) {
 // The scatter items' lists for the kernels that queue them, or none: then
 // scatter_stage makes them.
 static ScatterLists scatter_lists(const krr_wf *wf, bool inline_lists) {
-    return inline_lists ? ScatterLists{wf->scatter_lists, wf->scatter_class_counts(), wf->params.rr} : ScatterLists{};
+    return inline_lists ? ScatterLists{wf->scatter_lists, wf->scatter_class_counts(), wf->params.rr,
+                                       wf->medium ? nullptr : wf->q(Q_SHADOW).count}
+                        : ScatterLists{};
 }
 
 // Whether render() has the kernels that queue scatter items list them: at a
@@ -3056,7 +3070,8 @@ static int scatter_stage(krr_wf *wf, int depth, cudaStream_t st, bool to_tracker
         KRR_CUDA(launch_ordered(k_scatter_classify, wf->grid, wf->block, st, wf->scene, wf->q(Q_SCATTER), wf->ps,
                                 wf->params.rr, wf->scatter_lists, wf->scatter_class_counts()));
     KRR_CUDA(launch_ordered(k_scatter_process, wf->grid, wf->block, st, wf->scene, wf->q(Q_SCATTER), wf->scatter_lists,
-                                                     wf->scatter_class_counts(), wf->scatter_blocks_done(), wf->q(cur ^ 1),
+                                                     wf->scatter_class_counts(), wf->scatter_blocks_done(),
+                                                     listed && !wf->medium ? wf->q(cur).count : nullptr, wf->q(cur ^ 1),
                                                      wf->q(Q_SHADOW), tracked, wf->ps, wf->params.nee,
                                                      wf->params.rr, resident_grid(wf, 3), wf->err()));
     KRR_CUDA(cudaGetLastError());
@@ -3223,12 +3238,13 @@ extern "C" int krr_wf_render(krr_wf *wf, float *d_out, void *stream) {
     const bool pair = wf->params.nee && wf->medium && !split && wf->accel.levels == 1;
     for (int s = 0; s < wf->params.spp; ++s) {
         for (int64_t p0 = 0; p0 < wf->n; p0 += wf->qcap) {
-            KRR_TRY(krr_wf_reset_queues(wf, -1, stream));
-            KRR_TRY(camera_rays(wf, p0, std::min(wf->qcap, wf->n - p0), st));
+            KRR_TRY(camera_rays(wf, p0, std::min(wf->qcap, wf->n - p0), st, true));
             if (wf->nrc) KRR_CUDA(cudaMemsetAsync(wf->nrc_q_count(), 0, sizeof(int32_t), st));
             bool traced = false;
             for (int depth = 0;; ++depth) {
-                KRR_TRY(krr_wf_reset_queues(wf, depth, stream));
+                // without media the scatter and routing kernels empty the
+                // queues that they come after (scatter_stage, closest_stage)
+                if (wf->medium && depth > 0) KRR_TRY(krr_wf_reset_queues(wf, depth, stream));
                 KRR_TRY(closest_stage(wf, depth, st, traced, true));
                 if (wf->medium) {
                     {
