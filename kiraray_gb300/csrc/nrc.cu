@@ -527,6 +527,7 @@ namespace krr {
 
 NrcView nrc_view(const krr_nrc *n) { return NrcView{n->grid, n->mlp, n->table, n->weights}; }
 int64_t nrc_batch_size(const krr_nrc *n) { return n->cfg.batch_size; }
+int nrc_reserve_training(krr_nrc *n, int64_t records) { return ensure_capacity(n, records); }
 int32_t nrc_train_stride(const krr_nrc *n) { return n->cfg.train_pixel_stride; }
 float nrc_termination_spread(const krr_nrc *n) { return n->cfg.termination_spread; }
 const uint32_t *nrc_diverged_flag(const krr_nrc *n) { return n->err + 1; }

@@ -88,6 +88,7 @@ int nrc_query_device(krr_nrc *n, const float *d_inputs, const int32_t *d_count, 
                      float *d_out, cudaStream_t s);
 int nrc_train_device(krr_nrc *n, const float *d_inputs, const float *d_targets,
                      const int32_t *d_count, int64_t capacity, cudaStream_t s);
+int nrc_reserve_training(krr_nrc *n, int64_t records);   // buffers of a step of that many
 int64_t nrc_batch_size(const krr_nrc *n);
 // Byte offset of MLP parameter e (row-major [out][64] weights, layer by layer)
 // in the tensor-core kernels' canonical K-major tiles: 8 KB a layer, cores of

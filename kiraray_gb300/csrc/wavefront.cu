@@ -2129,7 +2129,9 @@ static int alloc_nrc_buffers(krr_wf *wf) {
     KRR_CUDA(cudaMemset(wf->nrc_rec_count, 0, (size_t)wf->nrc_slots * sizeof(int32_t)));
     KRR_CUDA(cudaMalloc(&wf->nrc_b_in, (size_t)batch * kNrcInputs * sizeof(float)));
     KRR_CUDA(cudaMalloc(&wf->nrc_b_t, (size_t)batch * 3 * sizeof(float)));
-    return KRR_OK;
+    // the step's own buffers now: a frame may be captured first, where nothing
+    // can be allocated
+    return wf->nrc_train ? nrc_reserve_training(wf->nrc, batch) : KRR_OK;
 }
 
 // End of a frame with training: build the batch from the recorded vertices
