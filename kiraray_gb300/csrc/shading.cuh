@@ -73,7 +73,7 @@ struct Pcg {
 // hexadecimal digit of the pixel's number the pair (A^n, sum) of 256 x digit x
 // 16^position steps, composed digit by digit, in place of a squaring for each
 // of the 30 bits of n.
-struct PcgJump {
+struct alignas(16) PcgJump {   // read by one 16-byte load
     uint64_t mult, plus;
 };
 struct PcgPixelJumps {
@@ -93,6 +93,7 @@ constexpr PcgPixelJumps make_pcg_pixel_jumps() {
     }
     return t;
 }
+static_assert(alignof(PcgPixelJumps) == 16 && sizeof(PcgJump) == 16, "advance_pixels reads 16 bytes at a time");
 static __device__ const PcgPixelJumps pcg_pixel_jumps = make_pcg_pixel_jumps();
 
 __device__ __forceinline__ void advance_pixels(Pcg &p, uint32_t pixel) {
