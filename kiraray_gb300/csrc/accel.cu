@@ -2029,7 +2029,12 @@ int accel_build_small(krr_accel *a, const float4 *d_boxes, int n, const TraceIns
     if (!*built) return KRR_OK;
     const auto t0 = std::chrono::steady_clock::now();
     static_assert(sizeof(SmallTreeResult) <= 64, "the result shares a small allocation");
-    if (a->small_cap < n || a->n_tris < 1) {
+    if (a->small_cap >= n && a->n_tris >= 1) {
+        // the live tree and records are overwritten: traces already launched,
+        // on whatever stream, end first (as the frees of a rebuild in new
+        // buffers wait for the device)
+        KRR_CUDA(cudaDeviceSynchronize());
+    } else {
         accel_free(a);
         a->small_cap = 0;
         KRR_CUDA(cudaMalloc(&a->d_scratch, 64));
