@@ -2048,9 +2048,8 @@ int accel_build_small(krr_accel *a, const float4 *d_boxes, int n, const TraceIns
     a->max_leaf = a->full_leaf = 1;
     a->builder = default_builder();
     a->collapse = a->treelets = 0;
-    static const cudaError_t attr = cudaFuncSetAttribute(k_small_tree, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)sizeof(SmallTreeShared));
-    KRR_CUDA(attr);
+    static OncePerDevice allowed;
+    KRR_CUDA(allow_shared(allowed, k_small_tree, sizeof(SmallTreeShared)));
     SmallTreeResult *d_res = reinterpret_cast<SmallTreeResult *>(a->d_small), res{};
     k_small_tree<<<1, kSmallTree, sizeof(SmallTreeShared), s>>>(d_boxes, n, a->builder != 0, a->d_nodes, a->d_tris,
                                                                 d_inst_new, d_inst, d_res);

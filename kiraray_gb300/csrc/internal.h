@@ -7,6 +7,7 @@
 #include <string>
 
 #include "../../include/krr_gb300.h"
+#include "per_device.h"
 
 namespace krr {
 
@@ -47,6 +48,18 @@ inline cudaError_t launch_ordered(void (*kernel)(P...), int grid, int block, cud
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// Raises a kernel's dynamic shared-memory limit, which belongs to the kernel
+// on one device: `done` is that kernel's own.
+template <typename... P>
+inline cudaError_t allow_shared(OncePerDevice &done, void (*kernel)(P...), size_t bytes) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return (cudaError_t)done(dev, [&] {
+        return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    });
 }
 
 }  // namespace krr

@@ -704,13 +704,9 @@ size_t nrc_tc_bwd_smem_bytes(int layers) {
 int nrc_backward_tc(const NrcMlp &mlp, int dx_cols, const float *d_out, const float *d_targets, float loss_scale,
                     const __nv_bfloat16 *acts, const int32_t *d_count, int64_t cap, const uint8_t *packed,
                     float *d_dx0, float *d_dw, float *d_loss, uint32_t *err, cudaStream_t s) {
-    static bool configured = false;
-    size_t smem = nrc_tc_bwd_smem_bytes(mlp.layers);
-    if (!configured) {
-        KRR_CUDA(cudaFuncSetAttribute(k_nrc_backward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)nrc_tc_bwd_smem_bytes(kNrcTcBwdLayers)));
-        configured = true;
-    }
+    const size_t smem = nrc_tc_bwd_smem_bytes(mlp.layers);
+    static OncePerDevice allowed;   // for the deepest network, whatever this one's depth
+    KRR_CUDA(allow_shared(allowed, k_nrc_backward_tc, nrc_tc_bwd_smem_bytes(kNrcTcBwdLayers)));
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -725,13 +721,9 @@ int nrc_backward_tc(const NrcMlp &mlp, int dx_cols, const float *d_out, const fl
 int nrc_forward_tc(const NrcGrid &g, const NrcMlp &mlp, const float *d_in, const int32_t *d_count,
                    int64_t cap, const __nv_bfloat16 *table, const uint8_t *packed, float *d_out, int out_stride,
                    __nv_bfloat16 *acts, uint32_t *err, cudaStream_t s) {
-    static bool configured = false;
-    size_t smem = nrc_tc_smem_bytes(mlp.layers);
-    if (!configured) {   // for the deepest network, whatever this one's depth
-        KRR_CUDA(cudaFuncSetAttribute(k_nrc_forward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)nrc_tc_smem_bytes(kNrcMaxLayers)));
-        configured = true;
-    }
+    const size_t smem = nrc_tc_smem_bytes(mlp.layers);
+    static OncePerDevice allowed;   // for the deepest network, whatever this one's depth
+    KRR_CUDA(allow_shared(allowed, k_nrc_forward_tc, nrc_tc_smem_bytes(kNrcMaxLayers)));
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
