@@ -201,7 +201,7 @@ int accel_update_instances(krr_accel *a, const float *inst_xf, cudaStream_t s);
 int launch_trace_instanced(const krr_accel *a, const TraceLaunch &l, int mode, cudaStream_t s);
 InstancedView instanced_view(const krr_accel *a);
 // Object-space triangles (9 floats) of n triangles of a mesh's arrays.
-int geometry_triangles(const float *d_pos, const uint32_t *d_idx, int64_t n, float *d_out, cudaStream_t s);
+int geometry_triangles(const float4 *d_vert, const uint32_t *d_idx, int64_t n, float *d_out, cudaStream_t s);
 // Reads and clears the traversal error flags (device int at d_err) after the
 // stream's work; KRR_ERR_OVERFLOW if a ray was cut off by the stack limit.
 int take_trace_errors(int *d_err, cudaStream_t s, uint32_t *out_flags);

@@ -218,14 +218,17 @@ k_trace_two_level_p(InstancedView v, TraceLaunch L) {
     }
 }
 
-// Object-space triangles of geometry g (mesh arrays) in [begin, end).
-__global__ void k_geometry_triangles(const float *__restrict__ pos, const uint32_t *__restrict__ idx,
+// Object-space triangles of a mesh: two float4 a vertex, its position first.
+__global__ void k_geometry_triangles(const float4 *__restrict__ vert, const uint32_t *__restrict__ idx,
                                      int64_t n, float *out) {
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= n) return;
     for (int k = 0; k < 3; ++k) {
         const uint32_t vi = idx[3 * t + k];
-        for (int c = 0; c < 3; ++c) out[9 * t + 3 * k + c] = pos[3 * vi + c];
+        const float4 p = vert[2 * (size_t)vi];
+        out[9 * t + 3 * k] = p.x;
+        out[9 * t + 3 * k + 1] = p.y;
+        out[9 * t + 3 * k + 2] = p.z;
     }
 }
 
@@ -489,9 +492,9 @@ int launch_trace_instanced(const krr_accel *a, const TraceLaunch &l, int mode, c
     return KRR_OK;
 }
 
-int geometry_triangles(const float *d_pos, const uint32_t *d_idx, int64_t n, float *d_out, cudaStream_t s) {
+int geometry_triangles(const float4 *d_vert, const uint32_t *d_idx, int64_t n, float *d_out, cudaStream_t s) {
     if (n == 0) return KRR_OK;
-    k_geometry_triangles<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_pos, d_idx, n, d_out);
+    k_geometry_triangles<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_vert, d_idx, n, d_out);
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }

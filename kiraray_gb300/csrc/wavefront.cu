@@ -378,7 +378,7 @@ __device__ Surf prepare_surface(const DevScene &s, float b1, float b2, uint32_t 
     V3 b = normalize(cross(n, t));
     o.u = 0.f;
     o.v = 0.f;
-    if (M.uv) {
+    if (M.has_uv) {
         o.u = c0.z * b0 + c1.z * b1 + c2.z * b2;
         o.v = c0.w * b0 + c1.w * b1 + c2.w * b2;
     }
@@ -430,9 +430,14 @@ __device__ __forceinline__ void light_triangle(const DevScene &s, const DevLight
     i0 = M->idx[3 * l.prim];
     i1 = M->idx[3 * l.prim + 1];
     i2 = M->idx[3 * l.prim + 2];
-    p0 = V3{M->pos[3 * i0], M->pos[3 * i0 + 1], M->pos[3 * i0 + 2]};
-    p1 = V3{M->pos[3 * i1], M->pos[3 * i1 + 1], M->pos[3 * i1 + 2]};
-    p2 = V3{M->pos[3 * i2], M->pos[3 * i2 + 1], M->pos[3 * i2 + 2]};
+    p0 = f3(__ldg(M->vert + 2 * (size_t)i0));
+    p1 = f3(__ldg(M->vert + 2 * (size_t)i1));
+    p2 = f3(__ldg(M->vert + 2 * (size_t)i2));
+}
+
+__device__ __forceinline__ V3 vertex_normal(const DevMesh &M, uint32_t i) {
+    const float4 b = __ldg(M.vert + 2 * (size_t)i + 1);
+    return V3{__ldg(&M.vert[2 * (size_t)i].w), b.x, b.y};
 }
 
 // Triangle::area, src/core/shape.h:29-38 (world-space vertices)
@@ -509,9 +514,9 @@ __device__ LightSample sample_li(const DevScene &s, const DevLight &l, float u0,
     const DevInstance *I;
     const DevMesh *M;
     light_triangle(s, l, p0, p1, p2, i0, i1, i2, I, M);
-    V3 n0{M->nrm[3 * i0], M->nrm[3 * i0 + 1], M->nrm[3 * i0 + 2]};
-    V3 n1{M->nrm[3 * i1], M->nrm[3 * i1 + 1], M->nrm[3 * i1 + 2]};
-    V3 n2{M->nrm[3 * i2], M->nrm[3 * i2 + 1], M->nrm[3 * i2 + 2]};
+    const V3 n0 = vertex_normal(*M, i0);
+    const V3 n1 = vertex_normal(*M, i1);
+    const V3 n2 = vertex_normal(*M, i2);
     V3 b = uniform_sample_triangle(u0, u1);
     V3 p = p0 * b.x + p1 * b.y + p2 * b.z;
     V3 n = normalize(cross(p1 - p0, p2 - p0));
@@ -1978,7 +1983,8 @@ __global__ void k_flatten(const DevScene s, int n_inst, float *out, int64_t n_tr
         uint32_t prim = (uint32_t)g - I.prim_offset;
         for (int k = 0; k < 3; ++k) {
             uint32_t vi = M.idx[3 * prim + k];
-            float x = M.pos[3 * vi], y = M.pos[3 * vi + 1], z = M.pos[3 * vi + 2];
+            const V3 p = f3(M.vert[2 * (size_t)vi]);
+            const float x = p.x, y = p.y, z = p.z;
             for (int r = 0; r < 3; ++r) {
                 const float *m = I.xf + 4 * r;
                 float acc = __fmul_rn(m[0], x);
@@ -2044,7 +2050,7 @@ int stage_grid(const krr_wf *wf, int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(g, (int64_t)sms * wf->blocks_per_sm));
 }
 
-// The shading copy of a mesh's vertices (DevMesh::vert).
+// A mesh's vertices as they stay on the device (DevMesh::vert).
 __global__ void k_pack_vertices(const float *__restrict__ pos, const float *__restrict__ nrm,
                                 const float *__restrict__ uv, int64_t n, float4 *out) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -2060,6 +2066,43 @@ int dev_upload(krr_wf *wf, T **dst, const T *src, size_t count) {
     KRR_CUDA(cudaMalloc(dst, count * sizeof(T)));
     wf->scene_allocs.push_back(*dst);
     KRR_CUDA(cudaMemcpy(*dst, src, count * sizeof(T), cudaMemcpyHostToDevice));
+    return KRR_OK;
+}
+
+// Device memory for a mesh's arrays on their way into the packed records.
+struct Staging {
+    float *d = nullptr;
+    int64_t floats = 0;
+    void release() {   // waits for the kernels that read it
+        cudaFree(d);
+        d = nullptr;
+        floats = 0;
+    }
+    ~Staging() { release(); }
+};
+
+// A mesh's positions, normals and texture coordinates into its records, all
+// on `st`: the arrays themselves do not stay on the device.
+int upload_vertices(krr_wf *wf, const krr_mesh_desc &m, Staging &stage, DevMesh &d, cudaStream_t st) {
+    const int64_t n = m.n_vertices;
+    KRR_CHECK_ARG(n >= 0, "negative vertex count");
+    d.has_uv = m.h_texcoords ? 1 : 0;
+    if (n == 0) return KRR_OK;
+    if (stage.floats < 8 * n) {
+        stage.release();
+        KRR_CUDA(cudaMalloc(&stage.d, 8 * n * sizeof(float)));
+        stage.floats = 8 * n;
+    }
+    float4 *vert = nullptr;
+    KRR_CUDA(cudaMalloc(&vert, 2 * n * sizeof(float4)));
+    wf->scene_allocs.push_back(vert);
+    float *pos = stage.d, *nrm = pos + 3 * n, *uv = d.has_uv ? nrm + 3 * n : nullptr;
+    KRR_CUDA(cudaMemcpyAsync(pos, m.h_positions, 3 * n * sizeof(float), cudaMemcpyHostToDevice, st));
+    KRR_CUDA(cudaMemcpyAsync(nrm, m.h_normals, 3 * n * sizeof(float), cudaMemcpyHostToDevice, st));
+    if (uv) KRR_CUDA(cudaMemcpyAsync(uv, m.h_texcoords, 2 * n * sizeof(float), cudaMemcpyHostToDevice, st));
+    k_pack_vertices<<<grid_for(n), kThreads, 0, st>>>(pos, nrm, uv, n, vert);
+    KRR_CUDA(cudaGetLastError());
+    d.vert = vert;
     return KRR_OK;
 }
 
@@ -2319,7 +2362,7 @@ static int build_two_level(krr_wf *wf, cudaStream_t st, bool update) {
         if (geom_of_mesh[m] < 0) {
             for (size_t g = 0; g < geom_mesh.size(); ++g) {
                 const DevMesh &o = meshes[geom_mesh[g]];
-                if (o.pos == meshes[m].pos && o.idx == meshes[m].idx &&
+                if (o.vert == meshes[m].vert && o.idx == meshes[m].idx &&
                     wf->h_mesh_tris[geom_mesh[g]] == wf->h_mesh_tris[m]) {
                     geom_of_mesh[m] = (int32_t)g;
                     break;
@@ -2343,7 +2386,7 @@ static int build_two_level(krr_wf *wf, cudaStream_t st, bool update) {
     int stat = KRR_OK;
     for (size_t g = 0; g < geom_mesh.size() && stat == KRR_OK; ++g)
         if (geom_mesh[g] >= 0)
-            stat = geometry_triangles(meshes[geom_mesh[g]].pos, meshes[geom_mesh[g]].idx,
+            stat = geometry_triangles(meshes[geom_mesh[g]].vert, meshes[geom_mesh[g]].idx,
                                       geom_begin[g + 1] - geom_begin[g], d_obj + 9 * geom_begin[g], st);
     InstancedInput in{d_obj, geom_begin.data(), (int)geom_mesh.size(), inst_geom.data(), xf.data(),
                       mask.data(), n};
@@ -2422,6 +2465,7 @@ extern "C" int krr_wf_set_scenes(krr_wf *wf, const krr_scene_desc *scenes, int32
 
     // meshes
     std::vector<DevMesh> meshes(mesh0[n_scenes]);
+    Staging staging;
     for (int p = 0; p < n_scenes; ++p) {
         const krr_scene_desc *sd = scenes + p;
         for (int i = 0; i < sd->n_meshes; ++i) {
@@ -2445,17 +2489,8 @@ extern "C" int krr_wf_set_scenes(krr_wf *wf, const krr_scene_desc *scenes, int32
             } else {
                 for (int64_t k = 0; k < 3 * m.n_triangles; ++k)
                     KRR_CHECK_ARG(m.h_indices[k] < (uint64_t)m.n_vertices, "mesh index out of range");
-                KRR_TRY(dev_upload(wf, const_cast<float **>(&d.pos), m.h_positions, 3 * m.n_vertices));
-                KRR_TRY(dev_upload(wf, const_cast<float **>(&d.nrm), m.h_normals, 3 * m.n_vertices));
-                if (m.h_texcoords) KRR_TRY(dev_upload(wf, const_cast<float **>(&d.uv), m.h_texcoords, 2 * m.n_vertices));
+                KRR_TRY(upload_vertices(wf, m, staging, d, st));
                 KRR_TRY(dev_upload(wf, const_cast<uint32_t **>(&d.idx), m.h_indices, 3 * m.n_triangles));
-                float4 *vert = nullptr;
-                KRR_CUDA(cudaMalloc(&vert, std::max<int64_t>(2 * m.n_vertices, 1) * sizeof(float4)));
-                wf->scene_allocs.push_back(vert);
-                d.vert = vert;
-                if (m.n_vertices > 0)
-                    k_pack_vertices<<<grid_for(m.n_vertices), kThreads, 0, st>>>(d.pos, d.nrm, d.uv, m.n_vertices, vert);
-                KRR_CUDA(cudaGetLastError());
             }
             d.material = m.material >= 0 ? m.material + mat0[p] : m.material;
             d.medium_inside = m.medium_inside >= 0 ? m.medium_inside + med0[p] : m.medium_inside;
@@ -2463,6 +2498,7 @@ extern "C" int krr_wf_set_scenes(krr_wf *wf, const krr_scene_desc *scenes, int32
             meshes[mesh0[p] + i] = d;
         }
     }
+    staging.release();
     // materials (src/scene/krrscene.cpp:208-227: specular alpha = 1 - roughness)
     std::vector<DevMaterial> mats(std::max(1, mat0[n_scenes]));
     for (int p = 0; p < n_scenes; ++p)

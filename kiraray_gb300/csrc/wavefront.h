@@ -8,14 +8,11 @@
 namespace krr {
 
 struct DevMesh {
-    const float *pos;       // float3, object space
-    const float *nrm;       // float3
-    const float *uv;        // float2 or nullptr
+    const float4 *vert;     // two per vertex, object space: position, normal.x | normal.yz, uv (0 without)
     const uint32_t *idx;    // uint3
-    const float4 *vert;     // shading's copy, two per vertex: pos, nrm.x | nrm.yz, uv (0 without)
     int32_t material;       // -1 = null material
     int32_t medium_inside, medium_outside;
-    int32_t pad;
+    int32_t has_uv;
 };
 
 struct DevInstance {
