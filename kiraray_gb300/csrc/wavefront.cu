@@ -2975,11 +2975,17 @@ static int nrc_evaluate_queries(krr_wf *wf, cudaStream_t st) {
 }
 
 // The scatter items' lists for the kernels that queue them, or none: then
-// scatter_stage makes them.
-static ScatterLists scatter_lists(const krr_wf *wf, bool inline_lists) {
-    return inline_lists ? ScatterLists{wf->scatter_lists, wf->scatter_class_counts(), wf->params.rr,
-                                       wf->medium ? nullptr : wf->q(Q_SHADOW).count}
-                        : ScatterLists{};
+// scatter_stage makes them.  In render() without media the routing kernel
+// also empties the shadow queue, at the last depth too.
+static ScatterLists scatter_lists(const krr_wf *wf, bool in_render, bool inline_lists) {
+    ScatterLists sl{};
+    if (inline_lists) {
+        sl.lists = wf->scatter_lists;
+        sl.counts = wf->scatter_class_counts();
+        sl.rr = wf->params.rr;
+    }
+    if (in_render && !wf->medium) sl.shadow_count = wf->q(Q_SHADOW).count;
+    return sl;
 }
 
 // Whether render() has the kernels that queue scatter items list them: at a
@@ -3033,7 +3039,7 @@ static int closest_stage(krr_wf *wf, int depth, cudaStream_t st, bool traced,
                                                       wf->q(Q_MISS), wf->q(Q_HIT_LIGHT), wf->q(Q_SCATTER),
                                                       wf->q(Q_MEDIUM_SAMPLE), wf->medium ? 1 : 0, wf->err(),
                                                       hook, wf->ps, inline_lights, wf->params.nee,
-                                                      scatter_lists(wf, in_render && lists_inline(wf, depth))));
+                                                      scatter_lists(wf, in_render, in_render && lists_inline(wf, depth))));
         KRR_CUDA(cudaGetLastError());
     }
     if (wf->nrc && !defer_cache) KRR_TRY(nrc_evaluate_queries(wf, st));
@@ -3707,7 +3713,7 @@ int launch_medium_sample(krr_wf *wf, int depth, cudaStream_t st, bool listed) {
                                                     wf->q((depth & 1) ^ 1), wf->q(Q_MISS),
                                                     wf->q(Q_HIT_LIGHT), wf->q(Q_SCATTER),
                                                     wf->q(Q_MEDIUM_SCATTER), wf->ps, order,
-                                                    wf->deal_cursor(0), scatter_lists(wf, listed), wf->err()));
+                                                    wf->deal_cursor(0), scatter_lists(wf, false, listed), wf->err()));
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
 }
