@@ -399,7 +399,11 @@ int krr_wf_update_instances(krr_wf *wf, int32_t n, const int32_t *h_indices,
 int krr_wf_rebuild_bvh(krr_wf *wf, void *stream);
 /* RenderPass::resize (integrator.cpp:181-184): reallocates queues. */
 int krr_wf_resize(krr_wf *wf, int32_t width, int32_t height);
-/* RenderPass::beginFrame (integrator.cpp:205-221). frame_index is 1-based. */
+/* RenderPass::beginFrame (integrator.cpp:205-221). frame_index is 1-based.
+ * The camera is read before the call returns.  Refused while the stream is
+ * being captured (krr_wf_capture_frame captures frames).  With up to 24 views
+ * the call does not wait for the stream: an error of work queued before it
+ * may then be reported by a later call. */
 int krr_wf_begin_frame(krr_wf *wf, int64_t frame_index, const krr_camera_desc *camera,
                        void *stream);
 /* RenderPass::render (integrator.cpp:223-267): writes float4 RGBA per pixel,

@@ -2884,6 +2884,12 @@ static int launch_begin_frame(krr_wf *wf, cudaStream_t st) {
 
 static int begin_frame_common(krr_wf *wf, int64_t frame_index, const krr_camera_desc *single,
                               const krr_view *views, int32_t n_views, cudaStream_t st) {
+    // a captured launch would replay this frame's index and cameras for ever:
+    // refused, whichever way they travel
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    KRR_CUDA(cudaStreamIsCapturing(st, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone)
+        return fail(KRR_ERR_CUDA, "begin_frame on a stream that is being captured: krr_wf_capture_frame captures frames");
     if (wf->n_views <= kSetupViews) {
         FrameSetup f{};
         KRR_TRY(fill_frame(wf, frame_index, single, views, n_views, f.views, &f.frame));
