@@ -555,13 +555,15 @@ __device__ __forceinline__ int view_of(const DevView *__restrict__ v, int n_view
 // A frame's constants and views as a launch argument, which the launch itself
 // copies: nothing to stage on the host and wait for, so that a frame is queued
 // while the one before it still runs (512x512 Cornell frame 428 and 417 us,
-// 241x135 frame 792 and 774 us).  24 views fit the 4 KB of arguments.
+// 241x135 frame 792 and 774 us).  A launch takes up to 32,764 bytes of
+// arguments here; 24 views, 4 KB, are what was measured, and frames of more
+// views keep the copies and the wait.
 constexpr int kSetupViews = 24;
 struct FrameSetup {
     FrameConst frame;
     DevView views[kSetupViews];
 };
-static_assert(sizeof(FrameSetup) <= 4000, "a launch takes 4 KB of arguments");
+static_assert(sizeof(FrameSetup) <= 32764, "a launch's arguments");
 
 __global__ void k_set_frame(const __grid_constant__ FrameSetup f, DevView *views, FrameConst *frame) {
     const int words = f.frame.n_views * (int)(sizeof(DevView) / 4);
