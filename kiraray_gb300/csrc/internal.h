@@ -36,6 +36,13 @@ enum DeviceError : uint32_t {
 // this hides the launch itself.  After anything that is not such a kernel
 // (copies, memsets, other launches) and for anything after it, the order is
 // the stream's as always.
+// The kernel's blocks may be resident while the one before it writes, so what
+// that one writes is not read-only for the kernel's life: it is read through
+// pointers that are not `const __restrict__`, and never by __ldg.  The
+// compiler may move those loads before stream_order() (a memory clobber does
+// not hold loads that it takes to be invariant) and serve them from the
+// read-only path.  Both are fine for what has been written before the kernel
+// before: the tree, the scene, the frame's views and constants.
 template <typename... P, typename... A>
 inline cudaError_t launch_ordered(void (*kernel)(P...), int grid, int block, cudaStream_t s, A &&...args) {
     cudaLaunchAttribute at{};

@@ -17,8 +17,9 @@ constexpr float k2Pi = 6.28318530717958647692f;
 constexpr float kRayEps = 1e-4f;   // KRR_RAY_EPS, src/core/raytracing.h:10
 
 // First statement of a kernel that launch_ordered() starts: the kernel before
-// it on the stream has ended and its writes are visible; and the kernel after
-// it may be brought up.
+// it on the stream has ended and its writes are visible, to loads that are not
+// of the invariant kind (launch_ordered); and the kernel after it may be
+// brought up.
 KRR_D void stream_order() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -755,7 +755,7 @@ __device__ __forceinline__ bool nrc_vertex(const NrcHook &h, const DevScene &s, 
 }
 
 // L[pixel] += throughput x max(cache, 0)
-__global__ void k_nrc_apply(const float *__restrict__ out, const float4 *__restrict__ meta,
+__global__ void k_nrc_apply(const float *out, const float4 *meta,
                             const int32_t *count, int cap, PixelState ps) {
     stream_order();
     int n = min(*count, cap);
@@ -890,7 +890,7 @@ __device__ __forceinline__ void list_item(const DevScene &s, int32_t material, i
 // sum gets the same terms in the same order as handleHit/handleMiss after
 // this stage.
 __global__ void __launch_bounds__(kThreads, 4)
-k_hit_process(DevScene s, Queue rq, const float4 *__restrict__ hits, Queue next, Queue miss,
+k_hit_process(DevScene s, Queue rq, const float4 *hits, Queue next, Queue miss,
               Queue hitl, Queue scat, Queue msq, int enable_medium, uint32_t *err, NrcHook hook,
               PixelState ps, int inline_lights, int nee, ScatterLists sl) {
     stream_order();
@@ -1134,7 +1134,7 @@ __global__ void k_scatter_classify(DevScene s, Queue scat, PixelState ps, float 
 // functions of their own (fewer instructions to fetch) on GB300: 27-30 us,
 // frames at 241x135 1,012 and 934 us, at 1920x1080 4.91 and 4.76 ms.
 __global__ void __launch_bounds__(kThreads, 3)
-k_scatter_process(DevScene s, Queue scat, const int32_t *__restrict__ lists,
+k_scatter_process(DevScene s, Queue scat, const int32_t *lists,
                   int32_t *counts, int32_t *blocks_done, int32_t *rays_done, Queue next, Queue shadow, Queue tracked,
                   PixelState ps, int nee, float rr, int resident, uint32_t *err) {
     stream_order();
@@ -1186,7 +1186,7 @@ k_scatter_process(DevScene s, Queue scat, const int32_t *__restrict__ lists,
 }
 
 // Radiance of unoccluded shadow rays (__raygen__Shadow, device.cu:92-100).
-__global__ void k_shadow_resolve(Queue shadow, const uint8_t *__restrict__ occluded, PixelState ps) {
+__global__ void k_shadow_resolve(Queue shadow, const uint8_t *occluded, PixelState ps) {
     stream_order();
     int n = min(*shadow.count, shadow.cap);   // an overflowed queue holds cap items
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1333,7 +1333,7 @@ __device__ __forceinline__ bool delta_track(const DevScene &s, const DevMedium &
 template <bool GREY>
 __global__ void __launch_bounds__(kThreads, 3)
 k_medium_sample(DevScene s, Queue msq, Queue next, Queue miss, Queue hitl, Queue scat,
-                Queue mscat, PixelState ps, const int32_t *__restrict__ order, int32_t *cursor, ScatterLists sl,
+                Queue mscat, PixelState ps, const int32_t *order, int32_t *cursor, ScatterLists sl,
                 uint32_t *err) {
     stream_order();
     int n = min(*msq.count, msq.cap);   // an overflowed queue holds cap items
@@ -1538,7 +1538,7 @@ __device__ __forceinline__ float4 shadow_trace(const InstancedView &iv, const fl
 template <int FMT, int LEVELS, bool GREY>
 __global__ void __launch_bounds__(kThreads, 3)
 k_shadow_tr(DevScene s, const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
-            InstancedView iv, Queue shadow, PixelState ps, const int32_t *__restrict__ order,
+            InstancedView iv, Queue shadow, PixelState ps, const int32_t *order,
             const float4 *first, int32_t *cursor, uint32_t *err, int *trace_err) {
     stream_order();
     int n = min(*shadow.count, shadow.cap);   // an overflowed queue holds cap items
