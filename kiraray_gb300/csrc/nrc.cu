@@ -484,17 +484,17 @@ int ensure_capacity(krr_nrc *n, int64_t cap) {
 // inputs in n->act and the output in n->out.
 // Queries read the inference copy of the parameters (the moving average when
 // ema_decay > 0), training the parameters themselves.
-// rgb (queries): the predictions go there, three floats a row, and the
-// tensor-core path keeps no buffers for them.
+// rgb (tensor-core queries): the predictions go there, three floats a row,
+// and no buffers are kept for them.
 int forward(krr_nrc *n, const float *d_inputs, const int32_t *d_count, int64_t cap, cudaStream_t s,
-            float *rgb = nullptr) {
-    const bool ema = rgb && n->ema_w;
+            bool query = false, float *rgb = nullptr) {
+    const bool ema = query && n->ema_w;
     const __nv_bfloat16 *table = ema ? n->ema_table_bf : n->table;
     const __nv_bfloat16 *weights = ema ? n->ema_weights : n->weights;
-    if (!rgb || !n->cfg.tensor_cores) KRR_TRY(ensure_capacity(n, cap));
+    if (!rgb) KRR_TRY(ensure_capacity(n, cap));
     if (n->cfg.tensor_cores)
         return nrc_forward_tc(n->grid, n->mlp, d_inputs, d_count, cap, table, ema ? n->ema_packed : n->packed,
-                              rgb ? rgb : n->out, rgb ? 3 : kNrcOutPad, rgb ? nullptr : n->act, n->err, s);
+                              rgb ? rgb : n->out, rgb ? 3 : kNrcOutPad, query ? nullptr : n->act, n->err, s);
     __nv_bfloat16 *A = n->act;
     k_encode<<<grid_for(cap), kThreads, 0, s>>>(n->grid, d_inputs, d_count, cap, table, A);
     KRR_CUDA(cudaGetLastError());
@@ -536,8 +536,12 @@ uint32_t *nrc_error_flags(krr_nrc *n) { return n->err; }
 int nrc_query_device(krr_nrc *n, const float *d_inputs, const int32_t *d_count, int64_t cap,
                      float *d_out, cudaStream_t s) {
     if (cap <= 0) return KRR_OK;
-    KRR_TRY(forward(n, d_inputs, d_count, cap, s, d_out));
-    if (n->cfg.tensor_cores) return KRR_OK;
+    // predictions that overlap the records (a query in place) are written when
+    // every record has been read: blocks take tiles of rows in no fixed order
+    const bool apart = d_out >= d_inputs + cap * kNrcInputs || d_inputs >= d_out + cap * 3;
+    const bool direct = n->cfg.tensor_cores && apart;
+    KRR_TRY(forward(n, d_inputs, d_count, cap, s, true, direct ? d_out : nullptr));
+    if (direct) return KRR_OK;
     k_write_rgb<<<grid_for(cap), kThreads, 0, s>>>(n->out, d_count, cap, d_out);
     KRR_CUDA(cudaGetLastError());
     return KRR_OK;
