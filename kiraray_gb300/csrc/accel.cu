@@ -1819,10 +1819,11 @@ static int build_ploc(int n, const float4 *leaf_lo, const float4 *leaf_hi, uint3
     return KRR_OK;
 }
 
-static int build_tree(krr_accel *a, const float *d_v, int64_t n, cudaStream_t s, int treelets) {
+static int build_tree(krr_accel *a, const float *d_v, int64_t n, cudaStream_t s, int treelets,
+                      int node_format) {
     KRR_CHECK_ARG(n >= 0 && n < (int64_t)0x7fffffff, "triangle count out of range");
     accel_free(a);
-    a->node_format = default_node_format();
+    a->node_format = node_format;
     a->max_leaf = default_max_leaf();
     a->full_leaf = std::max(a->max_leaf, default_full_leaf());
     a->n_tris = n;
@@ -2010,21 +2011,22 @@ static int build_tree(krr_accel *a, const float *d_v, int64_t n, cudaStream_t s,
 // Treelet passes of the BVHs built from now on (krr_set_bvh_treelets).
 static int g_treelets = 0;
 
-int accel_build(krr_accel *a, const float *d_v, int64_t n, cudaStream_t s) {
-    int st = build_tree(a, d_v, n, s, g_treelets);
+int accel_build(krr_accel *a, const float *d_v, int64_t n, cudaStream_t s, int node_format) {
+    if (node_format < 0) node_format = default_node_format();
+    int st = build_tree(a, d_v, n, s, g_treelets, node_format);
     // a restructured tree deeper than the traversal stack (possible on
     // degenerate input) is built again without restructuring
     if (st == KRR_ERR_OVERFLOW && g_treelets > 0 && a->max_depth > kTraversalStack)
-        st = build_tree(a, d_v, n, s, 0);
+        st = build_tree(a, d_v, n, s, 0, node_format);
     return st;
 }
 
 int small_tree_limit() { return kSmallTree; }
 
 int accel_build_small(krr_accel *a, const float4 *d_boxes, int n, const TraceInst *d_inst_new, TraceInst *d_inst,
-                      bool *built, cudaStream_t s) {
+                      int node_format, bool *built, cudaStream_t s) {
     // the settings that k_small_tree builds by
-    *built = n >= 1 && n <= kSmallTree && default_node_format() == 0 && default_max_leaf() == 1 &&
+    *built = n >= 1 && n <= kSmallTree && node_format == 0 && default_max_leaf() == 1 &&
              default_full_leaf() <= 1 && default_builder() != 1 && g_collapse == 0 && g_treelets == 0;
     if (!*built) return KRR_OK;
     const auto t0 = std::chrono::steady_clock::now();

@@ -119,7 +119,8 @@ int default_builder();    // krr_set_bvh_builder
 constexpr int kTraceThreads = 128;
 
 // Build from device world-space vertices (float3 x 3 per triangle).
-int accel_build(krr_accel *a, const float *d_vertices, int64_t n_tris, cudaStream_t stream);
+int accel_build(krr_accel *a, const float *d_vertices, int64_t n_tris, cudaStream_t stream,
+                int node_format = -1);   // -1: the format set for builds (krr_set_bvh_node_format)
 // New positions for the same triangles (same count and order): boxes refitted
 // bottom-up over the existing tree; the buffers keep their addresses.
 int accel_refit(krr_accel *a, const float *d_vertices, int64_t n_tris, cudaStream_t stream);
@@ -129,7 +130,7 @@ void accel_free(krr_accel *a);
 // *built false, and nothing done, for more than small_tree_limit() boxes or
 // build settings that only accel_build knows.
 int accel_build_small(krr_accel *a, const float4 *d_boxes, int n, const TraceInst *d_inst_new, TraceInst *d_inst,
-                      bool *built, cudaStream_t s);
+                      int node_format, bool *built, cudaStream_t s);
 int small_tree_limit();
 // Several BVHs, one per part of the triangles (part p holds the global ids
 // [part_begin[p], part_begin[p + 1])), in one node and triangle array: part

@@ -362,12 +362,14 @@ static int build_top_level_small(krr_accel *a, bool *built, cudaStream_t s) {
     KRR_CUDA(cudaGetLastError());
     a->h_inst.resize(n);
     a->h_inst_stale = true;
-    return accel_build_small(a->tlas, boxes, n, rec, a->d_inst, built, s);
+    return accel_build_small(a->tlas, boxes, n, rec, a->d_inst, a->blas->node_format, built, s);
 }
 
 // The top level over the instances' world boxes (each box given to the
 // builder as the degenerate triangle lo, hi, hi; the builder stores the
-// instance index as the triangle id).  Instance records alongside.
+// instance index as the triangle id).  Instance records alongside.  Both
+// levels have the geometries' node format, whatever is set for builds by now:
+// one traversal reads them.
 static int build_top_level(krr_accel *a, cudaStream_t s) {
     bool built = false;
     KRR_TRY(build_top_level_small(a, &built, s));
@@ -410,7 +412,7 @@ static int build_top_level(krr_accel *a, cudaStream_t s) {
     KRR_CUDA(cudaMalloc(&d_boxes, std::max<size_t>(boxes.size(), 9) * sizeof(float)));
     int st = cuda_status(cudaMemcpyAsync(d_boxes, boxes.data(), boxes.size() * sizeof(float),
                                          cudaMemcpyHostToDevice, s), "cudaMemcpyAsync", __FILE__, __LINE__);
-    if (st == KRR_OK) st = accel_build(a->tlas, d_boxes, n, s);
+    if (st == KRR_OK) st = accel_build(a->tlas, d_boxes, n, s, a->blas->node_format);
     cudaStreamSynchronize(s);
     cudaFree(d_boxes);
     if (st != KRR_OK) return st;
