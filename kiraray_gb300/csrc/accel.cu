@@ -723,7 +723,12 @@ __global__ void k_collapse(BinTree t, const CollapseItem *__restrict__ in, const
                 if (cost < best) { best = cost; bc = c; bs = s; }
             }
         }
-        if (bc < 0) break;
+        // no cost is a finite number (a NaN box, or one whose centre
+        // overflows): every child has a slot all the same
+        if (bc < 0) {
+            for (bc = 0; slot_of[bc] >= 0;) ++bc;
+            for (bs = 0; child_in_slot[bs] >= 0;) ++bs;
+        }
         slot_of[bc] = bs;
         child_in_slot[bs] = bc;
     }
