@@ -376,8 +376,8 @@ static int build_top_level(krr_accel *a, cudaStream_t s) {
     if (built) return KRR_OK;
     const int n = (int)a->inst_geom.size();
     std::vector<float> boxes(9 * (size_t)n);
-    a->h_inst.assign(n, TraceInst{});
-    a->h_inst_stale = false;
+    std::vector<TraceInst> records(n, TraceInst{});
+    bool infinite = false, number[3] = {n == 0, n == 0, n == 0};
     for (int i = 0; i < n; ++i) {
         const int g = a->inst_geom[i];
         const float *m = &a->inst_xf[12 * (size_t)i];
@@ -401,13 +401,21 @@ static int build_top_level(krr_accel *a, cudaStream_t s) {
             hi[r] += std::ldexp(mag, -20);
         }
         float *t = &boxes[9 * (size_t)i];
-        for (int r = 0; r < 3; ++r) { t[r] = lo[r]; t[3 + r] = hi[r]; t[6 + r] = hi[r]; }
-        TraceInst &I = a->h_inst[i];
+        for (int r = 0; r < 3; ++r) {
+            t[r] = lo[r]; t[3 + r] = hi[r]; t[6 + r] = hi[r];
+            infinite = infinite || std::isinf(lo[r]) || std::isinf(hi[r]);
+            number[r] = number[r] || !std::isnan(lo[r]) || !std::isnan(hi[r]);
+        }
+        TraceInst &I = records[i];
         invert_3x4(m, I.inv);
         I.blas_root = a->blas->roots.empty() ? 0u : a->blas->roots[g];
         I.id_delta = (uint32_t)(a->inst_first[i] - a->geom_begin[g]);
         I.mask = empty ? 0u : a->inst_mask[i];
     }
+    // bounds that accel_build refuses (it takes them over the numbers alone),
+    // before the tree that stands is given up
+    if (infinite || !number[0] || !number[1] || !number[2])
+        return fail(KRR_ERR_INVALID_ARGUMENT, "the instances' boxes are not finite");
     float *d_boxes = nullptr;
     KRR_CUDA(cudaMalloc(&d_boxes, std::max<size_t>(boxes.size(), 9) * sizeof(float)));
     int st = cuda_status(cudaMemcpyAsync(d_boxes, boxes.data(), boxes.size() * sizeof(float),
@@ -417,6 +425,8 @@ static int build_top_level(krr_accel *a, cudaStream_t s) {
     cudaFree(d_boxes);
     if (st != KRR_OK) return st;
     if (!a->d_inst) KRR_CUDA(cudaMalloc(&a->d_inst, std::max(1, n) * sizeof(TraceInst)));
+    a->h_inst.swap(records);
+    a->h_inst_stale = false;
     KRR_CUDA(cudaMemcpyAsync(a->d_inst, a->h_inst.data(), n * sizeof(TraceInst), cudaMemcpyHostToDevice, s));
     KRR_CUDA(cudaStreamSynchronize(s));
     return KRR_OK;
@@ -463,8 +473,13 @@ int accel_build_instanced(krr_accel *a, const InstancedInput &in, cudaStream_t s
 
 int accel_update_instances(krr_accel *a, const float *inst_xf, cudaStream_t s) {
     KRR_CHECK_ARG(a && a->levels == 2, "not a two-level structure");
-    std::memcpy(a->inst_xf.data(), inst_xf, a->inst_xf.size() * sizeof(float));
-    KRR_TRY(build_top_level(a, s));
+    std::vector<float> before(inst_xf, inst_xf + a->inst_xf.size());
+    a->inst_xf.swap(before);
+    const int st = build_top_level(a, s);
+    if (st != KRR_OK) {   // the structure keeps its transforms
+        a->inst_xf.swap(before);
+        return st;
+    }
     for (int k = 0; k < 3; ++k) { a->scene_lo[k] = a->tlas->scene_lo[k]; a->scene_hi[k] = a->tlas->scene_hi[k]; }
     return KRR_OK;
 }

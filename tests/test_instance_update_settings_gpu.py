@@ -37,3 +37,22 @@ def test_node_format_set_after_the_build(krr_lib, cuda, n, built, now):
             _check(acc, geos, insts, rays, "updated")
     finally:
         A.set_node_format(0)
+
+
+@pytest.mark.parametrize("n", [20, 1025])
+def test_refused_update_keeps_the_structure(krr_lib, cuda, n):
+    geos, insts = _instanced_scene(seed=8, n_inst=n)
+    acc = Accel.instanced(geos, insts)
+    rays = H.random_rays(2000, 5, box=5.0)
+    xf = np.stack([np.asarray(m, np.float32) for _, m in insts])
+    for value in (np.inf, -np.inf):
+        bad = xf.copy()
+        bad[7, 1, 3] = value
+        with pytest.raises(Exception, match="not finite"):
+            acc.update_instances(bad)
+        _check(acc, geos, insts, rays, "after a refused update")
+    with pytest.raises(Exception, match="not finite"):
+        acc.update_instances(np.full_like(xf, np.nan))
+    _check(acc, geos, insts, rays, "after a refused update")
+    acc.update_instances(xf)
+    _check(acc, geos, insts, rays, "updated again")
