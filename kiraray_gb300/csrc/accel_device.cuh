@@ -248,8 +248,9 @@ __device__ __forceinline__ void visit(const float4 *__restrict__ nodes, uint32_t
 }
 
 // One child of a compressed node, tested by one lane of a team of eight: the
-// box test of visit_node for the child in `slot` (same planes, same slack),
-// with the node's other words that the team needs.  A node is 80 bytes, so
+// box test of visit_node for the child in `slot` (the same planes 1024 + q,
+// offsets and slack, so that its bound holds here too), with the node's other
+// words that the team needs.  A node is 80 bytes, so
 // the team's loads of it fall into the same two or three sectors.
 __device__ __forceinline__ bool team_child(const float4 *__restrict__ nodes, uint32_t child, int slot,
                                            const RayPre &r, V3 inv, int oct, float tmax, uint32_t &meta,
@@ -268,19 +269,18 @@ __device__ __forceinline__ bool team_child(const float4 *__restrict__ nodes, uin
     const float adx = __uint_as_float((ew & 0xffu) << 23) * inv.x;
     const float ady = __uint_as_float(((ew >> 8) & 0xffu) << 23) * inv.y;
     const float adz = __uint_as_float(((ew >> 16) & 0xffu) << 23) * inv.z;
-    const float cx = fmaf(-32768.f, adx, (q0.x - r.o.x) * inv.x);
-    const float cy = fmaf(-32768.f, ady, (q0.y - r.o.y) * inv.y);
-    const float cz = fmaf(-32768.f, adz, (q0.z - r.o.z) * inv.z);
-    const float dx = adx * 0.00390625f, dy = ady * 0.00390625f, dz = adz * 0.00390625f;
+    const float cx = fmaf(-1024.f, adx, (q0.x - r.o.x) * inv.x);
+    const float cy = fmaf(-1024.f, ady, (q0.y - r.o.y) * inv.y);
+    const float cz = fmaf(-1024.f, adz, (q0.z - r.o.z) * inv.z);
     const float sx = fabsf(adx) * 0.015625f, sy = fabsf(ady) * 0.015625f, sz = fabsf(adz) * 0.015625f;
-    auto plane = [](uint32_t q) { return __uint_as_float(0x4B000000u | (q << 8)); };
+    auto plane = [](uint32_t q) { return __uint_as_float(0x44800000u | (q << 13)); };   // 1024 + q
     const float tlimit = tmax + fabsf(tmax) * 5e-7f;
-    const int t0 = __vimax3_s32(__float_as_int(fmaf(plane(nx), dx, cx - sx)),
-                                __float_as_int(fmaf(plane(ny), dy, cy - sy)),
-                                max(__float_as_int(fmaf(plane(nz), dz, cz - sz)), __float_as_int(r.tmin)));
-    const int t1 = __vimin3_s32(__float_as_int(fmaf(plane(fx), dx, cx + sx)),
-                                __float_as_int(fmaf(plane(fy), dy, cy + sy)),
-                                min(__float_as_int(fmaf(plane(fz), dz, cz + sz)), __float_as_int(tlimit)));
+    const int t0 = __vimax3_s32(__float_as_int(fmaf(plane(nx), adx, cx - sx)),
+                                __float_as_int(fmaf(plane(ny), ady, cy - sy)),
+                                max(__float_as_int(fmaf(plane(nz), adz, cz - sz)), __float_as_int(r.tmin)));
+    const int t1 = __vimin3_s32(__float_as_int(fmaf(plane(fx), adx, cx + sx)),
+                                __float_as_int(fmaf(plane(fy), ady, cy + sy)),
+                                min(__float_as_int(fmaf(plane(fz), adz, cz + sz)), __float_as_int(tlimit)));
     child_base = q1.x;
     tri_base = q1.y;
     imask = ew >> 24;
