@@ -390,7 +390,10 @@ int krr_wf_cache_box(krr_wf *wf, float *out_lo3, float *out_hi3);
  * row-major 3x4 transform h_transforms[12k..12k+11]; the world-space
  * triangles are re-flattened and the BVH's boxes refitted over its tree
  * (krr_accel_refit_triangles).  Device buffers stay in place: a captured
- * frame graph stays valid.  Frames equal those of a fresh scene. */
+ * frame graph stays valid.  With two levels the instance level is rebuilt
+ * (krr_accel_update_instances), in place up to 1,024 instances; with more a
+ * captured frame is dropped (capture again).  Frames equal those of a fresh
+ * scene. */
 int krr_wf_update_instances(krr_wf *wf, int32_t n, const int32_t *h_indices,
                             const float *h_transforms, void *stream);
 /* Full BVH build over the current instance transforms (restores the tree's

@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <tuple>
 #include <vector>
 
 #include "accel.h"
@@ -2784,8 +2785,21 @@ extern "C" int krr_wf_update_instances(krr_wf *wf, int32_t n, const int32_t *h_i
     KRR_CUDA(cudaStreamSynchronize(st));
     KRR_CUDA(cudaMemcpy(const_cast<DevInstance *>(wf->scene.instances), wf->h_instances.data(),
                         wf->h_instances.size() * sizeof(DevInstance), cudaMemcpyHostToDevice));
-    // a refit keeps every device buffer in place, so a captured frame stays valid
-    return rebuild_bvh(wf, st, true);
+    // a refit, and an instance tree of up to small_tree_limit() instances, keep
+    // every device buffer in place, so a captured frame stays valid; a larger
+    // instance tree is built in new buffers
+    const auto buffers = [&] {
+        const krr_accel &a = wf->accel;
+        return wf->levels == 2 && a.tlas ? std::make_tuple(a.tlas->d_nodes, a.tlas->d_tris, a.d_inst)
+                                         : std::make_tuple((float4 *)nullptr, (float4 *)nullptr, (TraceInst *)nullptr);
+    };
+    const auto before = buffers();
+    const int stat = rebuild_bvh(wf, st, true);
+    if (wf->graph && buffers() != before) {
+        cudaGraphExecDestroy(wf->graph);
+        wf->graph = nullptr;
+    }
+    return stat;
 }
 
 extern "C" int krr_wf_resize(krr_wf *wf, int32_t width, int32_t height) {
