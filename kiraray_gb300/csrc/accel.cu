@@ -2034,7 +2034,6 @@ int accel_build_small(krr_accel *a, const float4 *d_boxes, int n, const TraceIns
     *built = n >= 1 && n <= kSmallTree && node_format == 0 && default_max_leaf() == 1 &&
              default_full_leaf() <= 1 && default_builder() != 1 && g_collapse == 0 && g_treelets == 0;
     if (!*built) return KRR_OK;
-    const auto t0 = std::chrono::steady_clock::now();
     static_assert(sizeof(SmallTreeResult) <= 64, "the result shares a small allocation");
     if (a->small_cap >= n && a->n_tris >= 1) {
         // the live tree and records are overwritten: traces already launched,
@@ -2058,6 +2057,7 @@ int accel_build_small(krr_accel *a, const float4 *d_boxes, int n, const TraceIns
     static OncePerDevice allowed;
     KRR_CUDA(allow_shared(allowed, k_small_tree, sizeof(SmallTreeShared)));
     SmallTreeResult *d_res = reinterpret_cast<SmallTreeResult *>(a->d_small), res{};
+    const auto t0 = std::chrono::steady_clock::now();
     k_small_tree<<<1, kSmallTree, sizeof(SmallTreeShared), s>>>(d_boxes, n, a->builder != 0, a->d_nodes, a->d_tris,
                                                                 d_inst_new, d_inst, d_res);
     KRR_CUDA(cudaGetLastError());
