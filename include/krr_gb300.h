@@ -432,7 +432,7 @@ int krr_wf_set_megakernel_reorder(krr_wf *wf, int32_t reorder);
  * their items are taken class by class of estimated optical depth (the
  * ray's length inside the media's boxes times the largest sigma_t), so that
  * a warp's rays take similar numbers of null collisions.  The ordering costs
- * more than it saves on the 1024x1024 volume frame (11.1 against 10.1 ms),
+ * more than it saves on the 1024x1024 volume frame (6.0 against 5.3 ms),
  * hence off by default.  Frames are the same either way. */
 int krr_wf_set_media_order(krr_wf *wf, int32_t order);
 /* Order in which the camera stage queues each view's pixels (default 1):

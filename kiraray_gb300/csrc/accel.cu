@@ -806,10 +806,11 @@ __global__ void k_gather_tris(const float *__restrict__ v, const uint32_t *__res
 // move.  Up to kSmallTree boxes it is built by one block in shared memory:
 // the same Morton codes, radix tree and greedy collapse as above, a warp per
 // wide node (lane c holds child c) instead of a thread with its children in
-// local memory, no allocation and one round trip to the host.  501 instances
-// on GB300: 68 us with the records' kernel, 236 us of kernels and as much in
-// allocations and waits before; new transforms and 518,400 camera rays 1,028
-// and 495 us.
+// local memory, without an allocation.  501 instances on GB300: 68 us of
+// kernels, the records' among them, 236 us by the general builder; an update
+// of 200 or 1,024 instances 80 and 136 us, 465 and 660 us by the general
+// builder with its allocations and waits; new transforms of 501 instances and
+// 518,400 camera rays 463 us (1,025 us).
 constexpr int kSmallTree = 1024;
 
 struct SmallTreeShared {
@@ -1165,10 +1166,10 @@ __global__ void k_set_mask(float4 *tris, const uint32_t *leaf_of_prim, const uin
 // Every lane of a team carries the ray and a copy of its stack, so pushes
 // and pops need no exchange; child hits are exchanged by ballots and the
 // triangles' hits by a shuffle reduction to the smallest (t, id), the hit
-// the per-lane loop finds whatever its order.  On GB300, before and after:
-// 1,107 rays in the Cornell box 20.4 and 8.2 us; frames of the 10.9M-triangle
-// scene at 241x135 1,754 and 1,012 us, at 1920x1080 5,113 and 4,901 us; whole
-// sets of 2M rays the same within 2 %.  Teams of four lanes for five to eight
+// the per-lane loop finds whatever its order.  On GB300, without teams and
+// with them: 1,107 rays in the Cornell box 20.4 and 8.2 us; frames of the
+// 10.9M-triangle scene at 241x135 42 % less, at 1920x1080 4 %; whole sets of
+// 2M rays the same within 2 %.  Teams of four lanes for five to eight
 // rays (two children a lane) measured the same as none.
 constexpr int kTeamRays = 4;
 

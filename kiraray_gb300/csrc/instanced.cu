@@ -43,10 +43,10 @@ constexpr int kInstThreads = 128;
 constexpr uint32_t kTriGroupBit = 0x80000000u;   // stack entry: pending leaf group
 constexpr uint32_t kReturnBit = 0x40000000u;     // stack entry: back to the world ray
 
-// Eight blocks per SM (64 registers, the mixed variant spills 96 bytes):
-// 1.31 against 1.39 ms per 2.07M camera rays at six blocks (80 registers).
+// Eight blocks per SM (64 registers, 58 bytes spilled, 68 in the mixed
+// variant): 6 % less time for 2.07M camera rays than six blocks (80 registers).
 // The world ray and its inverse direction wait in shared memory while a lane
-// is inside an instance: 518,400 camera rays and an update 500 and 474 us.
+// is inside an instance: 5 % of 518,400 camera rays and an update.
 template <int MODE, int FMT>
 __global__ void __launch_bounds__(kInstThreads, 8)
 k_trace_two_level_p(InstancedView v, TraceLaunch L) {

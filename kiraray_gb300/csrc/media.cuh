@@ -16,8 +16,10 @@ namespace krr {
 // every spectrum of the walk (medium, transmittance, path probabilities) has
 // three equal channels.  One channel's operations give the bits that three
 // would, and a grey walk needs a third of them, with fewer registers.
-// 1024x1024 volume frame, whose medium is grey: 6.32 ms, and 6.76 ms with
-// three channels throughout but for the divisions and exponentials.
+// Against three channels throughout but for the divisions and exponentials,
+// the 1024x1024 volume frame, whose medium is grey, takes 6.5 % less time
+// (5.29 ms now; 5.98 ms with a coloured albedo, 5.71 ms with a coloured
+// sigma_t on a 128^3 grid).
 template <typename S>
 struct MediumProps {
     S sigma_a, sigma_s;
@@ -89,8 +91,8 @@ __device__ __forceinline__ float density_at(const DevMedium &m, V3 p) {
                 c[1][j][k] = half_to_float((uint16_t)(wd[2 * k + j] >> 16));
             }
         // below the first voxel of an axis: shifted, zeros outside.  A branch
-        // that next to no lookup takes (1024x1024 volume frame 6.09 ms, 6.19 ms
-        // with eight selects in each lookup)
+        // that next to no lookup takes (1.6 % of the 1024x1024 volume
+        // frame against eight selects in each lookup)
         if (sx | sy | sz) {
             if (sx)
 #pragma unroll
@@ -290,9 +292,9 @@ __device__ S sample_t_maj(const DevMedium &m, V3 o, V3 d, float tmax, Pcg &rng, 
     float tmin = 0.f;
     // One loop over the draws, whichever way they end: with the collisions of
     // a segment in a loop of their own the lanes of a warp waited at each of
-    // their segments for the one with the most collisions (1024x1024 volume
-    // frame 7.28 and 6.87 ms).  The step to the next segment stands in one
-    // place (6.33 ms with a second copy before the loop, 6.21 ms without).
+    // their segments for the one with the most collisions (5.6 % of the
+    // 1024x1024 volume frame).  The step to the next segment stands in one
+    // place (1.9 % against a second copy before the loop).
     bool fresh = true;
     while (true) {
         while (fresh) {   // to the next segment with a majorant in channel ch

@@ -298,9 +298,9 @@ __device__ __forceinline__ int push_slot_grouped(int32_t *count, int cap, uint32
 // Hands a queue's items to the resident warps of a tracking launch, 32 at a
 // time, fewer from a queue that is short of 32 for each: a warp takes as long
 // as its longest ray and both ways through each branch, so that rays spread
-// thin over otherwise idle warps end sooner (1024x1024 volume frame 6.87 ms
-// in queue order over all blocks, 6.76 ms dealt out; 8.1 ms with shares that
-// shrink with what is left, which fills too few lanes).  `cursor` is {next
+// thin over otherwise idle warps end sooner (1.6 % of the 1024x1024 volume
+// frame against queue order over all blocks; shares that shrink with what is
+// left cost 18 %: they fill too few lanes).  `cursor` is {next
 // item, warps done}, both 0 between launches.
 struct Deal {
     int32_t *cursor;
@@ -366,8 +366,8 @@ __device__ Surf prepare_surface(const DevScene &s, float b1, float b2, uint32_t 
     uint32_t i0 = M.idx[3 * prim], i1 = M.idx[3 * prim + 1], i2 = M.idx[3 * prim + 2];
     V3 wo = -normalize(ray_dir);
     o.wo = normalize(wo);
-    // a vertex in one 32-byte sector (1080p frame 4.50 and 4.47 ms, cached
-    // views 8x480x270 2.57 and 2.54 ms with three arrays of floats and with this)
+    // a vertex in one 32-byte sector (0.7 % of the 1080p frame and 1.2 % of
+    // the cached views 8x480x270 against three arrays of floats)
     const float4 a0 = __ldg(M.vert + 2 * (size_t)i0), a1 = __ldg(M.vert + 2 * (size_t)i1),
                  a2 = __ldg(M.vert + 2 * (size_t)i2);
     const float4 c0 = __ldg(M.vert + 2 * (size_t)i0 + 1), c1 = __ldg(M.vert + 2 * (size_t)i1 + 1),
@@ -555,8 +555,8 @@ __device__ __forceinline__ int view_of(const DevView *__restrict__ v, int n_view
 
 // A frame's constants and views as a launch argument, which the launch itself
 // copies: nothing to stage on the host and wait for, so that a frame is queued
-// while the one before it still runs (512x512 Cornell frame 428 and 417 us,
-// 241x135 frame 792 and 774 us).  A launch takes up to 32,764 bytes of
+// while the one before it still runs (2.6 % of the 512x512 Cornell frame,
+// 2.3 % of the 241x135 frame).  A launch takes up to 32,764 bytes of
 // arguments here; 24 views, 4 KB, are what was measured, and frames of more
 // views keep the copies and the wait.
 constexpr int kSetupViews = 24;
@@ -846,8 +846,8 @@ __device__ __forceinline__ V3 miss_radiance(const DevScene &s, const DevScenePar
 // kernels that queue its items when nothing happens between them (render()):
 // `lists` null leaves both to k_scatter_classify.  A path that the roulette
 // ends is then neither written to the queue nor read back, and a launch is
-// saved per bounce (512x512 Cornell frame 462 and 444 us, 1080p frame 4.47 and
-// 4.42 ms).
+// saved per bounce (3.9 % of the 512x512 Cornell frame, 1.1 % of the 1080p
+// frame).
 struct ScatterLists {
     int32_t *lists, *counts;
     float rr;
@@ -1123,7 +1123,7 @@ __global__ void k_scatter_classify(DevScene s, Queue scat, PixelState ps, float 
             list_item(s, sbits(scat.at(0, i).w), i, cap, lists, counts);
 }
 
-// Three blocks per SM (80 registers, 104 bytes spilled): 0.8 % faster per
+// Three blocks per SM (80 registers, 164 bytes spilled): 0.8 % faster per
 // 1080p frame than four blocks at 64 registers (236 bytes spilled).
 //
 // A launch of few items lasts as long as one item's chain of instructions,
@@ -1132,8 +1132,8 @@ __global__ void k_scatter_classify(DevScene s, Queue scat, PixelState ps, float 
 // item, one warp of a pair does its 32 items' light samples and the other
 // their BSDF samples; both take the sampler's state before the second stores
 // the new one.  With that, Bsdf::eval and the Fresnel and microfacet terms as
-// functions of their own (fewer instructions to fetch) on GB300: 27-30 us,
-// frames at 241x135 1,012 and 934 us, at 1920x1080 4.91 and 4.76 ms.
+// functions of their own (fewer instructions to fetch) on GB300: 22-30 us,
+// 7.7 % of the frame at 241x135 and 3.1 % at 1920x1080.
 __global__ void __launch_bounds__(kThreads, 3)
 k_scatter_process(DevScene s, Queue scat, const int32_t *lists,
                   int32_t *counts, int32_t *blocks_done, int32_t *rays_done, Queue next, Queue shadow, Queue tracked,
@@ -1330,7 +1330,7 @@ __device__ __forceinline__ bool delta_track(const DevScene &s, const DevMedium &
 // GREY: all of the pass's media are grey (krr_wf_set_scenes), so that every
 // walk is (the path probabilities start grey and only media could colour
 // them): less to fetch and to keep in registers, here and in k_shadow_tr
-// (1024x1024 volume frame 5.57 and 5.46 ms).
+// (2.0 % of the 1024x1024 volume frame).
 template <bool GREY>
 __global__ void __launch_bounds__(kThreads, 3)
 k_medium_sample(DevScene s, Queue msq, Queue next, Queue miss, Queue hitl, Queue scat,
@@ -3103,7 +3103,7 @@ static float4 *shadow_first_hits(const krr_wf *wf) {
 // stretch of bounce `depth`'s shadow rays in one launch, by the refilling
 // traversal instead of one ray's loop inside the tracker, where the lanes of a
 // warp wait for the longest; then the split and the tracking of the shadow
-// rays.  1024x1024 volume frame on GB300: 5.46 and 5.27 ms.
+// rays: 3.5 % of the 1024x1024 volume frame on GB300.
 static int track_shadow_and_trace_next(krr_wf *wf, int depth, cudaStream_t st) {
     {
         ProfScope prof(wf, PS_SHADOW_NEXT, st);
