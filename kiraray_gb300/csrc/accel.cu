@@ -1559,12 +1559,12 @@ static int launch_trace(const krr_accel *a, const TraceLaunch &l, cudaStream_t s
                        most <= (int64_t)grid * kTraceThreads;
     if (dealt && MODE < 2 && !l.d_count)
         grid = (int)std::min<int64_t>(grid, (l.n + kTraceThreads / 32 - 1) / (kTraceThreads / 32));
-    if (!dealt) KRR_CUDA(cudaMemsetAsync(l.counter, 0, sizeof(unsigned long long), s));
-    if (a->levels == 2) {
+    if (a->levels == 2) {   // clears the counter itself
         KRR_CHECK_ARG(!STATS, "the counter replay takes a one-level structure");
         KRR_CHECK_ARG(MODE != 3, "the pair launch takes a one-level structure");
         return launch_trace_instanced(a, lt, MODE, s);
     }
+    if (!dealt) KRR_CUDA(cudaMemsetAsync(l.counter, 0, sizeof(unsigned long long), s));
     const bool single = a->max_leaf == 1 && a->full_leaf == 1;
     if constexpr (MODE >= 2) {
         if (a->node_format == 1)
