@@ -237,9 +237,11 @@ int krr_accel_create_instanced(const float *h_geom_vertices, const int64_t *h_ge
                                krr_accel **out, void *stream);
 /* New object-to-world transforms for every instance (12 floats each): the
  * instance level is rebuilt, the geometry trees are kept (the OptiX IAS
- * update, optix.cpp:618-669).  Waits for the device: traces launched before
- * the call, on any stream, see the old transforms, those launched after it
- * the new ones.  Transforms that are refused leave the structure as it was. */
+ * update, optix.cpp:618-669).  Synchronous.  Traces launched before the call, on
+ * any stream, see the old transforms, those launched after it the new ones;
+ * where other streams than the given one have traced the structure since the
+ * last update, or a trace of it was captured, the call waits for the device.
+ * Transforms that are refused leave the structure as it was. */
 int krr_accel_update_instances(krr_accel *accel, const float *h_transforms, void *stream);
 /* The world-to-object 3x4 matrices the traversal uses (12 floats per
  * instance), for checking hits against an independent implementation. */

@@ -808,9 +808,9 @@ __global__ void k_gather_tris(const float *__restrict__ v, const uint32_t *__res
 // wide node (lane c holds child c) instead of a thread with its children in
 // local memory, without an allocation.  501 instances on GB300: 68 us of
 // kernels, the records' among them, 236 us by the general builder; an update
-// of 200 or 1,024 instances 80 and 136 us, 465 and 660 us by the general
+// of 200 or 1,024 instances 72 and 130 us, 465 and 660 us by the general
 // builder with its allocations and waits; new transforms of 501 instances and
-// 518,400 camera rays 463 us (1,025 us).
+// 518,400 camera rays 455 us (1,025 us).
 constexpr int kSmallTree = 1024;
 
 struct SmallTreeShared {
@@ -2030,17 +2030,17 @@ int accel_build(krr_accel *a, const float *d_v, int64_t n, cudaStream_t s, int n
 int small_tree_limit() { return kSmallTree; }
 
 int accel_build_small(krr_accel *a, const float4 *d_boxes, int n, const TraceInst *d_inst_new, TraceInst *d_inst,
-                      int node_format, bool *built, cudaStream_t s) {
+                      int node_format, bool in_flight, bool *built, cudaStream_t s) {
     // the settings that k_small_tree builds by
     *built = n >= 1 && n <= kSmallTree && node_format == 0 && default_max_leaf() == 1 &&
              default_full_leaf() <= 1 && default_builder() != 1 && g_collapse == 0 && g_treelets == 0;
     if (!*built) return KRR_OK;
     static_assert(sizeof(SmallTreeResult) <= 64, "the result shares a small allocation");
     if (a->small_cap >= n && a->n_tris >= 1) {
-        // the live tree and records are overwritten: traces already launched,
-        // on whatever stream, end first (as the frees of a rebuild in new
-        // buffers wait for the device)
-        KRR_CUDA(cudaDeviceSynchronize());
+        // the live tree and records are overwritten: traces launched on other
+        // streams end first (as the frees of a rebuild in new buffers wait
+        // for the device); those on this stream do anyway
+        if (in_flight) KRR_CUDA(cudaDeviceSynchronize());
     } else {
         accel_free(a);
         a->small_cap = 0;

@@ -33,6 +33,7 @@
 #include <stdint.h>
 
 #include "internal.h"
+#include "stream_use.h"
 
 namespace krr {
 // One instance of a two-level structure, as the traversal reads it.
@@ -93,6 +94,8 @@ struct krr_accel {
     // build_top_level (instanced.cu); h_inst is read back when it is asked for
     uint8_t *d_inst_in = nullptr;
     bool h_inst_stale = false;
+    // traversals of the instance tree since it was last written
+    mutable krr::StreamUse tree_use;
     // a tree of at most small_tree_limit() boxes (accel_build_small): boxes
     // its buffers hold, and its result's device copy
     int32_t small_cap = 0;
@@ -127,10 +130,11 @@ int accel_refit(krr_accel *a, const float *d_vertices, int64_t n_tris, cudaStrea
 void accel_free(krr_accel *a);
 // A tree over n boxes (d_boxes: lo, hi) in buffers that a later build of as
 // many keeps; d_inst takes d_inst_new's n records once the tree is built.
+// in_flight: the tree that stands may be read on other streams than s.
 // *built false, and nothing done, for more than small_tree_limit() boxes or
 // build settings that only accel_build knows.
 int accel_build_small(krr_accel *a, const float4 *d_boxes, int n, const TraceInst *d_inst_new, TraceInst *d_inst,
-                      int node_format, bool *built, cudaStream_t s);
+                      int node_format, bool in_flight, bool *built, cudaStream_t s);
 int small_tree_limit();
 // Several BVHs, one per part of the triangles (part p holds the global ids
 // [part_begin[p], part_begin[p + 1])), in one node and triangle array: part
@@ -200,7 +204,9 @@ int accel_build_instanced(krr_accel *a, const InstancedInput &in, cudaStream_t s
 // level is rebuilt, the geometry trees are kept.
 int accel_update_instances(krr_accel *a, const float *inst_xf, cudaStream_t s);
 int launch_trace_instanced(const krr_accel *a, const TraceLaunch &l, int mode, cudaStream_t s);
-InstancedView instanced_view(const krr_accel *a);
+// What a traversal on stream s reads: every launch that takes a view asks for
+// it here, so that an update knows which streams it has to wait for.
+InstancedView instanced_view(const krr_accel *a, cudaStream_t s);
 // Object-space triangles (9 floats) of n triangles of a mesh's arrays.
 int geometry_triangles(const float4 *d_vert, const uint32_t *d_idx, int64_t n, float *d_out, cudaStream_t s);
 // Reads and clears the traversal error flags (device int at d_err) after the

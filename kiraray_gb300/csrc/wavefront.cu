@@ -3795,7 +3795,7 @@ int launch_shadow_split(krr_wf *wf, cudaStream_t st, bool media_candidates, bool
     const Queue from = media_candidates ? Queue{wf->media_shadow, (int32_t)wf->qcap, wf->media_shadow_count()}
                                         : wf->q(Q_SHADOW);
     int *terr = wf->accel.d_scratch + 4;
-    const InstancedView iv = wf->accel.levels == 2 ? instanced_view(&wf->accel) : InstancedView{};
+    const InstancedView iv = wf->accel.levels == 2 ? instanced_view(&wf->accel, st) : InstancedView{};
 #define KRR_SHADOW_SPLIT(F, LV)                                                                        \
     KRR_CUDA(launch_ordered(k_shadow_split<F, LV>, wf->grid, wf->block, st, wf->scene, wf->accel.d_nodes, wf->accel.d_tris, iv, \
                                                           from, tracked, wf->ps,                     \
@@ -3812,7 +3812,7 @@ int launch_shadow_split(krr_wf *wf, cudaStream_t st, bool media_candidates, bool
 int launch_shadow_tracker(krr_wf *wf, cudaStream_t st, bool traced) {
     const Queue tracked = tracked_queue(wf);
     int *terr = wf->accel.d_scratch + 4;
-    const InstancedView iv = wf->accel.levels == 2 ? instanced_view(&wf->accel) : InstancedView{};
+    const InstancedView iv = wf->accel.levels == 2 ? instanced_view(&wf->accel, st) : InstancedView{};
     const int32_t *order = nullptr;
     KRR_TRY(work_order(wf, tracked, 1, st, &order));
 #define KRR_SHADOW_TR(F, LV)                                                                           \
